@@ -18,6 +18,9 @@
 // neighbour index, then one warp per support point that orders its segment
 // by entry number and adds the rows in that order, so every output channel
 // is summed in a fixed order -- no floating-point atomics.
+#include <climits>
+#include <cstdint>
+
 #include "fknn_common.cuh"
 #include "fknn_internal.h"
 #include "fknn_sort.cuh"
@@ -42,52 +45,134 @@ __device__ __forceinline__ bool entry_ok(int32_t t, int64_t n, int* status) {
 }  // namespace
 
 // ------------------------------------------------------------------ forward
+// Bound by the output stream: m*k*(c+3)*4 bytes written once, the feature
+// rows re-read from L2.
 
 // Rows of whole aligned float4s (no xyz, c % 4 == 0): a group of tpr lanes
 // (a power of two, tpr >= c/4 up to 32) copies one row, so a warp writes
 // 32/tpr consecutive rows as one contiguous run; the row loop is unrolled so
-// several independent gathers are in flight per thread.  Otherwise flat over
-// the output: thread t writes output float t.  Stores stream past L2
-// (st.global.cs): the output is written once and not re-read here.
+// several independent gathers are in flight per thread.  Stores stream past
+// L2 (st.global.cs): the output is written once and not re-read here.
 __global__ void __launch_bounds__(256)
     kg_forward(const float* __restrict__ feat, int64_t n, int c, const int32_t* __restrict__ idx,
-               int64_t rows, int k, const float* __restrict__ xyz,
-               const float* __restrict__ new_xyz, int with_xyz, int tpr,
-               float* __restrict__ out, int* status) {
+               int64_t rows, int tpr, float* __restrict__ out, int* status) {
   chain_wait();
-  const int off = with_xyz ? 3 : 0;
-  const int cw = c + off;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  if (tpr) {  // with_xyz == 0, c % 4 == 0
-    const int q4 = c >> 2;
-    const int sub = threadIdx.x & (tpr - 1);
-    const int64_t row_stride = stride / tpr;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int q4 = c >> 2;
+  const int sub = threadIdx.x & (tpr - 1);
+  const int64_t row_stride = stride / tpr;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-    for (int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / tpr;
-         r < rows; r += row_stride) {
-      const int32_t t = idx[r];
-      const bool ok = entry_ok(t, n, sub == 0 ? status : nullptr);
-      const float4* src = reinterpret_cast<const float4*>(feat + static_cast<int64_t>(t) * c);
-      float4* dst = reinterpret_cast<float4*>(out) + r * q4;
-      for (int q = sub; q < q4; q += tpr) __stcs(dst + q, ok ? __ldg(src + q) : zero);
-    }
-    return;
-  }
-  const int64_t words = rows * cw;
-  for (int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; w < words;
-       w += stride) {
-    const int64_t r = w / cw;
-    const int col = static_cast<int>(w - r * cw);
+  for (int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / tpr; r < rows;
+       r += row_stride) {
     const int32_t t = idx[r];
-    float v = 0.f;
-    if (entry_ok(t, n, col == 0 ? status : nullptr)) {
-      if (col < off)
-        v = __fsub_rn(xyz[3 * static_cast<int64_t>(t) + col], new_xyz[3 * (r / k) + col]);
-      else
-        v = __ldg(feat + static_cast<int64_t>(t) * c + (col - off));
+    const bool ok = entry_ok(t, n, sub == 0 ? status : nullptr);
+    const float4* src = reinterpret_cast<const float4*>(feat + static_cast<int64_t>(t) * c);
+    float4* dst = reinterpret_cast<float4*>(out) + r * q4;
+    for (int q = sub; q < q4; q += tpr) __stcs(dst + q, ok ? __ldg(src + q) : zero);
+  }
+}
+
+// Rows that are not whole float4s (the xyz part makes them c+3 floats wide):
+// a warp gathers R consecutive rows (R % 4 == 0, so the run starts 16-byte
+// aligned whatever the width) into its shared-memory slice -- 16-byte loads
+// when the feature rows allow it -- and stores the run as float4s.  One
+// word per thread, the row found by a 64-bit division, was bound by those
+// instructions instead: 3.2 million rows of 3 + 64 floats (858 MB written)
+// took 638 us; this takes 232 us (3.7 TB/s written; with streaming stores 271 us).
+__global__ void __launch_bounds__(256)
+    kg_forward_staged(const float* __restrict__ feat, int64_t n, int c,
+                      const int32_t* __restrict__ idx, int64_t rows, int k,
+                      const float* __restrict__ xyz, const float* __restrict__ new_xyz, int off,
+                      int R, int tpr, float* __restrict__ out, int* status) {
+  chain_wait();
+  extern __shared__ __align__(16) float kg_smem[];
+  const int lane = threadIdx.x & 31;
+  const int cw = c + off;
+  float* sm = kg_smem + static_cast<int64_t>(threadIdx.x >> 5) * R * cw;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  const int64_t groups = (rows + R - 1) / R;
+  int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  auto load_idx = [&](int64_t at) {
+    return lane < R && at * R + lane < rows ? __ldg(idx + at * R + lane) : -1;
+  };
+  int32_t t_next = load_idx(g);
+  for (; g < groups; g += warps) {
+    const int64_t r0 = g * R;
+    const int nr = rows - r0 < R ? static_cast<int>(rows - r0) : R;
+    int32_t t = t_next;
+    if (!entry_ok(t, n, status)) t = -1;
+    t_next = load_idx(g + warps);  // in flight while this run is gathered and stored
+    if (off) {  // R <= 8: one (row, axis) per lane
+      const int r = lane / 3, a = lane - 3 * r;
+      const int32_t tr = __shfl_sync(kFull, t, r);
+      if (r < nr) {
+        const int64_t i = static_cast<uint32_t>(r0 + r) / static_cast<uint32_t>(k);
+        sm[r * cw + a] = tr < 0 ? 0.f
+                                : __fsub_rn(__ldg(xyz + 3 * static_cast<int64_t>(tr) + a),
+                                            __ldg(new_xyz + 3 * i + a));
+      }
     }
-    __stcs(out + w, v);
+    if (tpr) {  // whole float4s of features: tpr lanes per row
+      const int q4 = c >> 2;
+      const int sub = lane & (tpr - 1);
+      const int step = 32 / tpr;
+#pragma unroll 4
+      for (int rr = 0; rr < R; rr += step) {
+        const int r = rr + lane / tpr;
+        const int32_t tr = __shfl_sync(kFull, t, r);
+        const float4* src = reinterpret_cast<const float4*>(feat + static_cast<int64_t>(tr) * c);
+        float* dst = sm + r * cw + off;
+        if (r < nr)
+          for (int q = sub; q < q4; q += tpr) {
+            const float4 v = tr < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(src + q);
+            dst[4 * q] = v.x;
+            dst[4 * q + 1] = v.y;
+            dst[4 * q + 2] = v.z;
+            dst[4 * q + 3] = v.w;
+          }
+      }
+    } else {
+      for (int r = 0; r < nr; ++r) {
+        const int32_t tr = __shfl_sync(kFull, t, r);
+        const float* src = feat + static_cast<int64_t>(tr) * c;
+        for (int q = lane; q < c; q += 32) sm[r * cw + off + q] = tr < 0 ? 0.f : __ldg(src + q);
+      }
+    }
+    __syncwarp();
+    const int words = nr * cw;
+    float* dst = out + r0 * cw;
+    for (int w = lane; w < (words >> 2); w += 32)
+      reinterpret_cast<float4*>(dst)[w] = reinterpret_cast<const float4*>(sm)[w];
+    if (lane < (words & 3)) dst[(words & ~3) + lane] = sm[(words & ~3) + lane];
+    __syncwarp();
+  }
+}
+
+// Any width and alignment: one warp per row, one word per lane.
+__global__ void __launch_bounds__(256)
+    kg_forward_rows(const float* __restrict__ feat, int64_t n, int c,
+                    const int32_t* __restrict__ idx, int64_t rows, int k,
+                    const float* __restrict__ xyz, const float* __restrict__ new_xyz, int off,
+                    float* __restrict__ out, int* status) {
+  chain_wait();
+  const int lane = threadIdx.x & 31;
+  const int cw = c + off;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+       r < rows; r += warps) {
+    const int32_t t = idx[r];
+    const bool ok = entry_ok(t, n, lane == 0 ? status : nullptr);
+    for (int col = lane; col < cw; col += 32) {
+      float v = 0.f;
+      if (ok) {
+        if (col < off)
+          v = __fsub_rn(xyz[3 * static_cast<int64_t>(t) + col], new_xyz[3 * (r / k) + col]);
+        else
+          v = __ldg(feat + static_cast<int64_t>(t) * c + (col - off));
+      }
+      __stcs(out + r * cw + col, v);
+    }
   }
 }
 
@@ -150,15 +235,21 @@ struct Vec<2> {
 
 // One warp per support point: its entries in ascending order, each row of
 // grad_out added channel by channel in that order.  V channels per lane (2
-// when the rows are whole float2s); the rows of four entries are loaded
-// before they are added, in order, so loads overlap.
-template <int V>
+// when the rows are whole float2s) and NC column blocks of 32*V channels, so
+// rows of up to 32*V*NC channels are read in one walk over the entries; the
+// rows of kRows entries are loaded before they are added, in order, so
+// kRows*NC loads are in flight per lane.  Bound by reading grad_out once: walking the
+// entries again for every 32 channels (NC = 1), 3.2 million rows of 3 + 64
+// floats (858 MB) took 321 us, one walk with four
+// rows in flight 296 us, with eight 218 us.
+template <int V, int NC>
 __global__ void __launch_bounds__(256)
     kg_support(const float* __restrict__ grad_out, int c, int with_xyz,
                const uint32_t* __restrict__ start, const uint32_t* __restrict__ seg, int64_t n,
                float* __restrict__ grad_feat, float* __restrict__ grad_xyz, int accumulate_xyz) {
   chain_wait();
   using VT = typename Vec<V>::T;
+  constexpr int kRows = 8;
   const int lane = threadIdx.x & 31;
   const int off = with_xyz ? 3 : 0;
   const int cw = c + off;
@@ -170,26 +261,31 @@ __global__ void __launch_bounds__(256)
     // walked by repeated selection of the next larger entry.
     uint32_t mine = kNoEntry;
     if (len <= 32) mine = warp_sort_u32(lane < static_cast<int>(len) ? seg[s + lane] : kNoEntry);
-    for (int c0 = 0; c0 < cw; c0 += 32 * V) {
-      const int col = c0 + lane * V;
-      const bool live = col < cw;
-      auto row = [&](uint32_t e) {
-        return *reinterpret_cast<const VT*>(grad_out + static_cast<int64_t>(e) * cw + col);
-      };
-      VT acc = Vec<V>::zero();
-      if (len <= 32) {
-        uint32_t r = 0;
-        for (; r + 4 <= len; r += 4) {
-          const uint32_t e0 = __shfl_sync(kFull, mine, r), e1 = __shfl_sync(kFull, mine, r + 1);
-          const uint32_t e2 = __shfl_sync(kFull, mine, r + 2), e3 = __shfl_sync(kFull, mine, r + 3);
-          if (live) {
-            const VT v0 = row(e0), v1 = row(e1), v2 = row(e2), v3 = row(e3);
-            acc = Vec<V>::add(Vec<V>::add(Vec<V>::add(Vec<V>::add(acc, v0), v1), v2), v3);
-          }
+    for (int c0 = 0; c0 < cw; c0 += 32 * V * NC) {
+      VT acc[NC];
+#pragma unroll
+      for (int b = 0; b < NC; ++b) acc[b] = Vec<V>::zero();
+      auto load = [&](uint32_t e, VT (&v)[NC]) {
+        const float* row = grad_out + static_cast<int64_t>(e) * cw;
+#pragma unroll
+        for (int b = 0; b < NC; ++b) {
+          const int col = c0 + (b * 32 + lane) * V;
+          v[b] = col < cw ? *reinterpret_cast<const VT*>(row + col) : Vec<V>::zero();
         }
-        for (; r < len; ++r) {
-          const uint32_t e = __shfl_sync(kFull, mine, r);
-          if (live) acc = Vec<V>::add(acc, row(e));
+      };
+      auto add = [&](const VT (&v)[NC]) {
+#pragma unroll
+        for (int b = 0; b < NC; ++b) acc[b] = Vec<V>::add(acc[b], v[b]);
+      };
+      if (len <= 32) {
+        for (uint32_t r = 0; r < len; r += kRows) {
+          VT v[kRows][NC];
+#pragma unroll
+          for (int u = 0; u < kRows; ++u)
+            if (r + u < len) load(__shfl_sync(kFull, mine, r + u), v[u]);
+#pragma unroll
+          for (int u = 0; u < kRows; ++u)
+            if (r + u < len) add(v[u]);
         }
       } else {
         uint32_t last = 0;
@@ -200,43 +296,74 @@ __global__ void __launch_bounds__(256)
             if ((r == 0 || v > last) && v < best) best = v;
           }
           best = __reduce_min_sync(kFull, best);
-          if (live) acc = Vec<V>::add(acc, row(best));
+          VT v[NC];
+          load(best, v);
+          add(v);
           last = best;
         }
       }
-      if (!live) continue;
-      if constexpr (V == 1) {
-        if (col < off) {
-          if (grad_xyz) {
-            float* g = grad_xyz + 3 * p + col;
-            *g = accumulate_xyz ? __fadd_rn(*g, acc) : acc;
+#pragma unroll
+      for (int b = 0; b < NC; ++b) {
+        const int col = c0 + (b * 32 + lane) * V;
+        if (col >= cw) continue;
+        if constexpr (V == 1) {
+          if (col < off) {
+            if (grad_xyz) {
+              float* g = grad_xyz + 3 * p + col;
+              *g = accumulate_xyz ? __fadd_rn(*g, acc[b]) : acc[b];
+            }
+          } else {
+            grad_feat[p * c + (col - off)] = acc[b];
           }
-        } else {
-          grad_feat[p * c + (col - off)] = acc;
+        } else {  // no xyz part: channel col of the row is channel col of feat
+          *reinterpret_cast<VT*>(grad_feat + p * c + col) = acc[b];
         }
-      } else {  // no xyz part: channel col of the row is channel col of feat
-        *reinterpret_cast<VT*>(grad_feat + p * c + col) = acc;
       }
     }
   }
 }
 
-// grad_new_xyz[i] = -sum_j over valid entries of the xyz part of row (i, j).
+// grad_new_xyz[i] = -sum_j over valid entries of the xyz part of row (i, j),
+// j ascending.  A warp takes 32 / kp queries (kp: k rounded up to a power of
+// two, at most 32), one row per lane, so the 12 bytes of 32 rows are in
+// flight at once; each query's lane 0 then subtracts its rows in order.  One
+// thread per query, one row in flight at a time, took 85 us for 3.2 million
+// rows of 268 bytes; this takes 70 us.
 __global__ void __launch_bounds__(256)
     kg_query(const float* __restrict__ grad_out, int c, const int32_t* __restrict__ idx,
-             int64_t m, int k, int64_t n, float* __restrict__ grad_new_xyz, int accumulate) {
+             int64_t m, int k, int64_t n, int kp, float* __restrict__ grad_new_xyz,
+             int accumulate) {
   chain_wait();
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (kp - 1);
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t i = warp * (32 / kp) + lane / kp;
   const int cw = c + 3;
   float g[3] = {0.f, 0.f, 0.f};
-  for (int j = 0; j < k; ++j) {
-    const int32_t t = idx[i * k + j];
-    if (t < 0 || t >= n) continue;
-    const float* row = grad_out + (i * k + j) * cw;
+  for (int j0 = 0; j0 < k; j0 += kp) {
+    const int j = j0 + sub;
+    float v[3] = {0.f, 0.f, 0.f};
+    bool ok = false;
+    if (i < m && j < k) {
+      const int32_t t = idx[i * k + j];
+      ok = t >= 0 && t < n;
+      if (ok) {
+        const float* row = grad_out + (i * k + j) * cw;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) g[a] = __fsub_rn(g[a], row[a]);
+        for (int a = 0; a < 3; ++a) v[a] = __ldg(row + a);
+      }
+    }
+    const uint32_t valid = __ballot_sync(kFull, ok) >> (lane - sub);
+    for (int r = 0; r < kp; ++r) {
+      const bool take = (valid >> r) & 1u;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float x = __shfl_sync(kFull, v[a], r, kp);
+        if (take) g[a] = __fsub_rn(g[a], x);
+      }
+    }
   }
+  if (i >= m || sub != 0) return;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     grad_new_xyz[3 * i + a] = accumulate ? __fadd_rn(grad_new_xyz[3 * i + a], g[a]) : g[a];
@@ -299,18 +426,29 @@ int run_group_forward(const GroupArgs& g, void* ws, size_t ws_bytes, cudaStream_
   const int64_t rows = g.m * g.k;
   int nl = 0;
   if (rows > 0) {
-    const int cw = g.c + (g.with_xyz ? 3 : 0);
-    const bool vec4 = !g.with_xyz && g.c % 4 == 0 &&
-                      reinterpret_cast<uintptr_t>(g.feat) % 16 == 0 &&
-                      reinterpret_cast<uintptr_t>(g.out) % 16 == 0;
-    int tpr = 0;  // lanes per row of the float4 path
-    if (vec4) {
+    const int off = g.with_xyz ? 3 : 0, cw = g.c + off;
+    const bool out16 = reinterpret_cast<uintptr_t>(g.out) % 16 == 0;
+    const bool feat4 = g.c % 4 == 0 && reinterpret_cast<uintptr_t>(g.feat) % 16 == 0;
+    int tpr = 0;  // lanes per row of float4 features
+    if (feat4) {
       tpr = 1;
       while (tpr < 32 && tpr < g.c / 4) tpr <<= 1;
     }
-    const int64_t words = vec4 ? rows * tpr : rows * cw;
-    launch_chained(kg_forward, capped_blocks(words), 256, 0, s, g.feat, g.n, g.c, g.idx, rows, g.k,
-                   g.xyz, g.new_xyz, g.with_xyz, tpr, g.out, &b.meta->status);
+    // Rows per warp of the staged path: 8 while a CTA's eight slices stay
+    // within 40 KB (five CTAs per SM), 4 up to the 48 KB that need no opt-in;
+    // wider rows amortise the per-row work by themselves.
+    const int R = cw <= 160 ? 8 : (cw <= 384 ? 4 : 0);
+    if (feat4 && out16 && !off) {
+      launch_chained(kg_forward, capped_blocks(rows * tpr), 256, 0, s, g.feat, g.n, g.c, g.idx,
+                     rows, tpr, g.out, &b.meta->status);
+    } else if (out16 && R && rows <= INT32_MAX) {
+      launch_chained(kg_forward_staged, capped_warp_blocks(ceil_div(rows, R)), 256,
+                     sizeof(float) * 8 * R * cw, s, g.feat, g.n, g.c, g.idx, rows, g.k, g.xyz,
+                     g.new_xyz, off, R, tpr, g.out, &b.meta->status);
+    } else {
+      launch_chained(kg_forward_rows, capped_warp_blocks(rows), 256, 0, s, g.feat, g.n, g.c, g.idx,
+                     rows, g.k, g.xyz, g.new_xyz, off, g.out, &b.meta->status);
+    }
     ++nl;
   }
   e = cudaGetLastError();
@@ -350,17 +488,25 @@ int run_group_backward(const GroupArgs& g, void* ws, size_t ws_bytes, cudaStream
     const bool v2 = !g.with_xyz && g.c % 2 == 0 &&
                     reinterpret_cast<uintptr_t>(g.grad_out) % 8 == 0 &&
                     reinterpret_cast<uintptr_t>(g.grad_feat) % 8 == 0;
-    if (v2)
-      launch_chained(kg_support<2>, capped_warp_blocks(g.n), 256, 0, s, g.grad_out, g.c, 0, b.start,
-                     b.seg, g.n, g.grad_feat, nullptr, 0);
-    else
-      launch_chained(kg_support<1>, capped_warp_blocks(g.n), 256, 0, s, g.grad_out, g.c, g.with_xyz,
+    const int cw = g.c + (g.with_xyz ? 3 : 0);
+    const int blocks = static_cast<int>(ceil_div(cw, v2 ? 64 : 32));  // of channels
+    auto support = [&](auto kernel) {
+      launch_chained(kernel, capped_warp_blocks(g.n), 256, 0, s, g.grad_out, g.c, g.with_xyz,
                      b.start, b.seg, g.n, g.grad_feat, g.grad_xyz, g.accumulate_xyz);
+    };
+    if (v2)
+      blocks <= 1 ? support(kg_support<2, 1>) : support(kg_support<2, 2>);
+    else
+      blocks <= 1   ? support(kg_support<1, 1>)
+      : blocks == 2 ? support(kg_support<1, 2>)
+                    : support(kg_support<1, 3>);
     ++nl;
   }
   if (g.with_xyz && g.grad_new_xyz && g.m > 0) {
-    launch_chained(kg_query, static_cast<int>(ceil_div(g.m, 256)), 256, 0, s, g.grad_out, g.c,
-                   g.idx, g.m, g.k, g.n, g.grad_new_xyz, g.accumulate_new_xyz);
+    int kp = 1;
+    while (kp < 32 && kp < g.k) kp <<= 1;
+    launch_chained(kg_query, static_cast<int>(ceil_div(g.m, 256 / kp)), 256, 0, s, g.grad_out, g.c,
+                   g.idx, g.m, g.k, g.n, kp, g.grad_new_xyz, g.accumulate_new_xyz);
     ++nl;
   }
   e = cudaGetLastError();

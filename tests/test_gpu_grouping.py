@@ -98,3 +98,34 @@ def test_knn_query_and_group_full_size(fk):
     assert torch.equal(grouped, want)
     plain, idx2 = fk.knn_query_and_group(feat, xyz, offs, idx=idx, with_xyz=False)
     assert torch.equal(plain, feat[il]) and idx2 is idx
+
+
+@pytest.mark.parametrize("with_xyz", [False, True])
+@pytest.mark.parametrize("m,k,c,shift", [
+    (1, 1, 1, 0), (3, 5, 3, 0), (37, 16, 4, 0), (37, 16, 4, 1), (61, 33, 29, 0), (41, 7, 64, 0),
+    (41, 7, 64, 1), (50, 8, 67, 0), (33, 3, 96, 0), (33, 3, 128, 0), (29, 9, 157, 0),
+    (29, 9, 160, 0), (13, 5, 381, 0), (13, 5, 384, 0), (13, 5, 388, 0)])
+def test_row_widths_and_alignments(fk, m, k, c, shift, with_xyz):
+    """Every gather path (float4 rows, staged runs, row by row) at the edges
+    of its widths, with feature rows off the 16-byte alignment (shift) and
+    padding entries; gradients against FP64 sums of at most m*k FP32 terms."""
+    rng = np.random.default_rng(m * 1000 + c)
+    n = 53
+    idx = rng.integers(-1, n, (m, k)).astype(np.int32)
+    z = {"idx": idx, "feat": rng.standard_normal((n, c)).astype(np.float32),
+         "xyz": rng.random((n, 3), dtype=np.float32),
+         "new_xyz": rng.random((m, 3), dtype=np.float32),
+         "grad_out": rng.standard_normal((m, k, c + 3 * with_xyz)).astype(np.float32),
+         "with_xyz": np.bool_(with_xyz), "separate": np.bool_(True)}
+    flat = torch.empty(n * c + shift, device=DEV)
+    feat = flat[shift:].view(n, c)
+    feat.copy_(T(z["feat"]))
+    feat.requires_grad_(True)
+    xyz, new = T(z["xyz"], True), T(z["new_xyz"], True)
+    out = fk.grouping(T(idx), feat, xyz, new, with_xyz=with_xyz)
+    want_out, want = grouping_f64(z)
+    assert np.array_equal(out.detach().cpu().numpy(), want_out.astype(np.float32))
+    out.backward(T(z["grad_out"]))
+    got = {"feat": feat.grad, "xyz": xyz.grad, "new_xyz": new.grad}
+    for key in ("feat",) + (("xyz", "new_xyz") if with_xyz else ()):
+        assert rel(got[key].cpu().numpy(), want[key]) <= 1e-5
