@@ -5,16 +5,33 @@
 
 namespace fknn {
 
+// Order of two 64-bit list keys.  A key (distance bits << 32 | index, or the
+// empty key) is the bit pattern of a non-negative double that is no NaN, so
+// its order as a double is its order as an integer, and the comparison is one
+// FP64 instruction instead of two on the integer ALU, the pipe that bounds
+// the networks.
+__device__ __forceinline__ bool key_less(uint64_t a, uint64_t b) {
+  return __longlong_as_double(static_cast<long long>(a)) <
+         __longlong_as_double(static_cast<long long>(b));
+}
+
 // Ascending sorting networks (comparator counts 1, 5, 19, 60,
 // 185, 531 for 2..64 keys).  8 and 16 keys use published minimum-size
 // networks; larger sizes sort both halves and join them with Batcher's
 // odd-even merge.  Each network was checked with the 0-1 principle (all
 // 2^n binary inputs for n <= 16, all pairs of sorted binary halves for the
 // merges).
-template <int KCAP, typename T>
-__device__ __forceinline__ void cas_up(T (&L)[KCAP], int i, int j) {
-  const T a = L[i], b = L[j];
-  const bool sw = b < a;
+template <int KCAP>
+__device__ __forceinline__ void cas_up(uint32_t (&L)[KCAP], int i, int j) {
+  const uint32_t a = L[i], b = L[j];
+  L[i] = min(a, b);
+  L[j] = max(a, b);
+}
+
+template <int KCAP>
+__device__ __forceinline__ void cas_up(uint64_t (&L)[KCAP], int i, int j) {
+  const uint64_t a = L[i], b = L[j];
+  const bool sw = key_less(b, a);
   L[i] = sw ? b : a;
   L[j] = sw ? a : b;
 }

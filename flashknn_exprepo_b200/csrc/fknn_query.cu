@@ -14,18 +14,18 @@
 //     groups, one query per lane.  Each group's 27 runs are staged into the
 //     warp's shared-memory tile by non-multicast cp.async.bulk copies that
 //     complete on the warp's mbarrier.  Each group's candidates are then
-//     counting-sorted (32 buckets of squared distance) by distance to the centroid of the
-//     group's queries, so every lane fills its list with near candidates
-//     first: the first KCAP candidates are sorted by a sorting network, the
-//     rest go through a branch-free insertion network only when some lane
-//     improves (warp vote), and a lane stops at the first bucket whose lower
-//     distance bound exceeds its current K-th distance (triangle
-//     inequality, with a safety margin for FP32 rounding);
+//     counting-sorted (32 buckets of squared distance) by distance to the
+//     centroid of the group's queries, so every lane meets near candidates
+//     first and stops at the first bucket whose lower distance bound exceeds
+//     its current K-th distance (triangle inequality, with a safety margin
+//     for FP32 rounding).  Lists of 8 and more take the candidates in blocks
+//     sorted and merged as 32-bit keys (select_blocks); shorter ones insert
+//     them one by one when some lane improves (warp vote);
 //   * chunked item: one group with more candidates than a tile; G lanes per
 //     query split its candidates, streamed tile by tile, and the G partial
 //     lists are merged with xor-shuffle bitonic merges;
-//   * lists hold packed u64 keys (distance bits << 32 | index), so ordering
-//     is exact including ties; rows are written straight to the caller's
+//   * results come from packed u64 keys (distance bits << 32 | index), so
+//     ordering is exact including ties; rows are written straight to the caller's
 //     row / index space.
 #include <algorithm>
 #include <cfloat>
@@ -38,38 +38,53 @@
 
 namespace fknn {
 
-constexpr uint64_t kEmpty = ~0ull;
+// Larger than every key (the distance bits of a key are those of a finite
+// float) and, read as a double, +inf: see key_less.
+constexpr uint64_t kEmpty = 0x7ff0000000000000ull;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr int kBuckets = 32;
 constexpr int kMaxOrderedGroup = 4096;  // queries: larger chunked groups keep record order
 
-// Per-group scratch of the current packed item (shared memory, per warp).
-struct GroupSlot {
+// One group of the current packed item (shared memory, per warp).
+struct __align__(16) GroupSlot {
   int seg;    // first tile slot of the group's candidates
   int len;    // number of candidates
   int a, b;   // the group's query range inside the item (query-record positions)
-  float cx, cy, cz;  // centroid of those queries
-  float inv_w2;      // 1 / bucket width in squared distance
-  float eps;         // absolute margin of the early-exit bound
-  int pad0, pad1, pad2;
 };
-static_assert(sizeof(GroupSlot) == 48, "GroupSlot layout");
+
+// A lane's group while its query is scanned.
+struct LaneGroup {
+  int len;                   // candidates to scan
+  const uint16_t* srt;       // their tile positions in bucket order
+  const uint16_t* bstart;    // first of every bucket
+  float inv_w2;              // 1 / bucket width in squared distance
+  float rq;                  // distance of the query to the group's centroid
+  float eps;                 // absolute margin of the early-exit bound
+};
 
 // Staging buffers per warp (the autotuner's depth axis: 1 or 2).
 constexpr int kMaxStaging = 2;
+
+// Slots for the sorted tile positions of an item's groups: each group's start
+// is a multiple of 8, so eight positions are one 16-byte load.
+__host__ __device__ constexpr size_t sorted_slots(int T) {
+  return static_cast<size_t>(T) + 8 * kMaxGroupsPerItem;
+}
 
 // Bytes of one warp's shared-memory region: `depth` staging buffers of T
 // records (tile, group slots, flag) and one set of sort scratch.
 __host__ __device__ constexpr size_t warp_smem_bytes(int T, int depth) {
   return ((static_cast<size_t>(depth) *
-               (static_cast<size_t>(T) * 16 + kMaxGroupsPerItem * sizeof(GroupSlot) + 16) +
-           static_cast<size_t>(T) * 4 + kMaxGroupsPerItem * (kBuckets + 1) * 2 + 32 +
-           kBuckets * 4 + 127) /
+               (static_cast<size_t>(T) * 16 + kMaxGroupsPerItem * sizeof(GroupSlot) + 32) +
+           sorted_slots(T) * 2 + static_cast<size_t>(T) * 2 +
+           kMaxGroupsPerItem * (kBuckets + 1) * 2 + kBuckets * 4 + 127) /
           128) *
          128;
 }
 
-__device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
+__device__ __forceinline__ uint64_t key_min(uint64_t a, uint64_t b) {
+  return key_less(a, b) ? a : b;
+}
 
 __device__ __forceinline__ uint64_t make_key(float d, float w) {
   return (static_cast<uint64_t>(__float_as_uint(d)) << 32) |
@@ -83,11 +98,11 @@ template <int KCAP>
 __device__ __forceinline__ void list_insert(uint64_t (&L)[KCAP], uint64_t x) {
 #pragma unroll
   for (int j = KCAP - 1; j >= 1; --j) {
-    const bool cj = x < L[j];
-    const bool cm = x < L[j - 1];
+    const bool cj = key_less(x, L[j]);
+    const bool cm = key_less(x, L[j - 1]);
     L[j] = cj ? (cm ? L[j - 1] : x) : L[j];
   }
-  L[0] = x < L[0] ? x : L[0];
+  L[0] = key_min(x, L[0]);
 }
 
 // The same network over the upper half only: valid when x does not belong
@@ -96,8 +111,8 @@ template <int KCAP>
 __device__ __forceinline__ void list_insert_upper(uint64_t (&L)[KCAP], uint64_t x) {
 #pragma unroll
   for (int j = KCAP - 1; j >= KCAP / 2; --j) {
-    const bool cj = x < L[j];
-    const bool cm = x < L[j - 1];
+    const bool cj = key_less(x, L[j]);
+    const bool cm = key_less(x, L[j - 1]);
     L[j] = cj ? (cm ? L[j - 1] : x) : L[j];
   }
 }
@@ -105,7 +120,7 @@ __device__ __forceinline__ void list_insert_upper(uint64_t (&L)[KCAP], uint64_t 
 template <int KCAP>
 __device__ __forceinline__ void cas(uint64_t (&L)[KCAP], int i, int j, bool ascending) {
   const uint64_t a = L[i], b = L[j];
-  const bool sw = ascending ? (b < a) : (a < b);
+  const bool sw = ascending ? key_less(b, a) : key_less(a, b);
   L[i] = sw ? b : a;
   L[j] = sw ? a : b;
 }
@@ -116,7 +131,7 @@ __device__ __forceinline__ void cas(uint64_t (&L)[KCAP], int i, int j, bool asce
 template <int KCAP>
 __device__ __forceinline__ void insert_one(uint64_t (&L)[KCAP], uint64_t x) {
   if constexpr (KCAP >= 8) {
-    if (__all_sync(kFull, x >= L[KCAP / 2 - 1])) {
+    if (__all_sync(kFull, !key_less(x, L[KCAP / 2 - 1]))) {
       list_insert_upper<KCAP>(L, x);
       return;
     }
@@ -144,15 +159,15 @@ __device__ __forceinline__ uint64_t shfl_xor_u64(uint64_t v, int mask) {
 template <int KCAP>
 __device__ __forceinline__ void merge_with_lane(uint64_t (&L)[KCAP], int mask) {
   if constexpr (KCAP == 1) {
-    L[0] = umin64(L[0], shfl_xor_u64(L[0], mask));
+    L[0] = key_min(L[0], shfl_xor_u64(L[0], mask));
   } else {
 #pragma unroll
     for (int j = 0; j < KCAP / 2; ++j) {
       const uint64_t a = L[j], b = L[KCAP - 1 - j];
       const uint64_t pa = shfl_xor_u64(b, mask);  // partner's L[KCAP-1-j]
       const uint64_t pb = shfl_xor_u64(a, mask);  // partner's L[j]
-      L[j] = umin64(a, pa);
-      L[KCAP - 1 - j] = umin64(b, pb);
+      L[j] = key_min(a, pa);
+      L[KCAP - 1 - j] = key_min(b, pb);
     }
     bitonic_clean_ascending<KCAP>(L);
   }
@@ -205,20 +220,147 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // distance to the centroid: a candidate in bucket b lies at least
 // sqrt(b*w2) from the centroid, hence at least sqrt(b*w2) - rq from the
 // query; buckets with b*w2 > (rq + sqrt(thr))^2 (plus margins) are skipped.
-template <int KCAP>
-__device__ __forceinline__ int stop_position(const uint64_t (&L)[KCAP], const GroupSlot& s,
-                                             float rq, const uint16_t* bstart) {
-  const uint64_t last = L[KCAP - 1];
-  if (last == kEmpty) return s.len;
+__device__ __forceinline__ int stop_position(float kth, const LaneGroup& s) {
   // m * rsqrt(m) is within a few ulp of sqrt(m), far inside the 1e-4 margin;
   // m >= FLT_MIN keeps a K-th distance of 0 (a query on a support point) or
   // a subnormal one bounded from above, and +inf gives NaN, which skips no
   // bucket
-  const float m = fmaxf(__uint_as_float(static_cast<uint32_t>(last >> 32)), FLT_MIN);
-  const float reach = rq + m * rsqrtf(m) * 1.0001f + s.eps;
+  const float m = fmaxf(kth, FLT_MIN);
+  const float reach = s.rq + m * rsqrtf(m) * 1.0001f + s.eps;
   const float lim = reach * reach * s.inv_w2;
   if (!(lim < static_cast<float>(kBuckets - 1))) return s.len;
-  return bstart[static_cast<int>(lim) + 1];
+  return s.bstart[static_cast<int>(lim) + 1];
+}
+
+// The next item of the queue, in lane 0 (item_of() gives it to every lane),
+// so that the atomic is in flight while the warp finishes its current item.
+__device__ __forceinline__ int pop_item(Meta* meta) {
+  return (threadIdx.x & 31) == 0 ? atomicAdd(&meta->queue_head, 1) : 0;
+}
+__device__ __forceinline__ int item_of(int popped) { return __shfl_sync(kFull, popped, 0); }
+
+// Order-preserving 32-bit keys of the packed scan: the squared distance's
+// bits with the low ones replaced by the candidate's position in its group's
+// sorted list, so a compare-exchange is a min and a max.
+constexpr uint32_t kNone32 = ~0u;
+
+// Merges the ascending block X into the ascending list L, keeping the KCAP
+// smallest; dropped = the smallest key ever left out.
+template <int KCAP, int B>
+__device__ __forceinline__ void merge_block(uint32_t (&L)[KCAP], const uint32_t (&X)[B],
+                                            uint32_t& dropped) {
+  constexpr int o = KCAP - B;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    const uint32_t l = L[o + j], x = X[B - 1 - j];
+    L[o + j] = min(l, x);
+    dropped = min(dropped, max(l, x));
+  }
+#pragma unroll
+  for (int st = KCAP / 2; st > 0; st >>= 1) {
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j)
+      if ((j & st) == 0) cas_up<KCAP>(L, j, j + st);
+  }
+}
+
+// The lane's KCAP smallest candidates as exact keys (distance bits << 32 |
+// index), ascending; entries from k on may be left out.
+//
+// Bound by instruction issue.  The scan sorts blocks of B candidates as
+// 32-bit keys and merges each block into the list (a minimum and a maximum
+// per compare-exchange), in place of one warp-wide 64-bit insertion per
+// accepted candidate of any lane: 309 -> about 200 warp instructions per
+// query at K=16.  The first block goes through the same loop as the rest (no
+// separate fill): the code the warps share has to stay small, since straight
+// copies of it made instruction fetch the first stall (2.8 of 10 cycles per
+// instruction).  With the sort's reworked loops the whole call over the
+// 16-cloud batch (1.46 million queries, K=16) went from 861 to 614 us, over
+// 700 thousand queries at K=32 from 880 to 573 us, over 300 thousand at K=64
+// from 1182 to 607 us.  The keys
+// drop the low 9 or 10 bits of the distance, so the exact keys of the list
+// are computed at the end and neighbours that the truncation left in the
+// wrong order are exchanged; a lane whose k-th entry shares its truncated
+// distance with a candidate it left out collects the candidates of that one
+// truncated distance again, with exact keys.
+template <int KCAP, typename DistBits>
+__device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGroup& g, int k,
+                                              uint32_t pos_mask, uint32_t cut_lim,
+                                              DistBits& dist_bits, Meta* meta, bool pop,
+                                              int& popped) {
+  constexpr int B = KCAP <= 16 ? 8 : 16;
+  const uint16_t* srt = g.srt;
+  uint32_t L[KCAP];
+  uint32_t dropped = kNone32, last = kNone32;
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) L[j] = kNone32;
+  int stop = g.len;
+#pragma unroll 1
+  for (int t0 = 0; __any_sync(kFull, t0 < stop); t0 += B) {
+    uint32_t X[B];
+#pragma unroll
+    for (int h = 0; h < B; h += 8) {  // eight positions per 16-byte load
+      const bool live = t0 + h < stop;
+      uint4 p = make_uint4(0u, 0u, 0u, 0u);
+      if (live) p = *reinterpret_cast<const uint4*>(srt + t0 + h);
+      const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float4 c;
+        const uint32_t d = dist_bits((u & 1) ? pw[u >> 1] >> 16 : pw[u >> 1] & 0xffffu, c);
+        X[h + u] = live && d <= cut_lim ? (d & ~pos_mask) | static_cast<uint32_t>(t0 + h + u)
+                                        : kNone32;
+      }
+    }
+    sort_network<B, 0, B>(X);
+    if (__any_sync(kFull, X[0] < last)) {
+      merge_block<KCAP, B>(L, X, dropped);
+      last = L[KCAP - 1];
+      if (k < KCAP) {
+#pragma unroll
+        for (int j = 0; j < KCAP - 1; ++j)
+          if (j == k - 1) last = L[j];
+      }
+      if (last != kNone32) stop = min(stop, stop_position(__uint_as_float(last | pos_mask), g));
+    } else {
+      dropped = min(dropped, X[0]);
+    }
+  }
+  if (pop) popped = pop_item(meta);
+  // Exact keys; entries of an ambiguous k-th truncated distance stay out.
+  const bool ambiguous = last != kNone32 && ((dropped ^ last) & ~pos_mask) == 0u;
+  const uint32_t limit = ambiguous ? last & ~pos_mask : kNone32;
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) {
+    E[j] = kEmpty;
+    if (L[j] < limit) {
+      float4 c;
+      const uint32_t d = dist_bits(srt[L[j] & pos_mask], c);
+      E[j] = make_key(__uint_as_float(d), c.w);
+    }
+  }
+  while (true) {
+    bool sorted = true;
+#pragma unroll
+    for (int j = 0; j + 1 < KCAP; ++j) sorted = sorted && !key_less(E[j + 1], E[j]);
+    if (__all_sync(kFull, sorted)) break;
+#pragma unroll
+    for (int j = 0; j + 1 < KCAP; j += 2) cas_up<KCAP>(E, j, j + 1);
+#pragma unroll
+    for (int j = 1; j + 1 < KCAP; j += 2) cas_up<KCAP>(E, j, j + 1);
+  }
+  if (__any_sync(kFull, ambiguous)) {
+    const int end = ambiguous ? stop : 0;
+    for (int t = 0; __any_sync(kFull, t < end); ++t) {
+      uint64_t x = kEmpty;
+      if (t < end) {
+        float4 c;
+        const uint32_t d = dist_bits(srt[t], c);
+        if (d <= cut_lim && (d & ~pos_mask) == limit) x = make_key(__uint_as_float(d), c.w);
+      }
+      if (__any_sync(kFull, x != kEmpty)) list_insert<KCAP>(E, x);
+    }
+  }
 }
 
 template <typename IdxT, int KCAP, bool EXACT>
@@ -271,14 +413,20 @@ __device__ __forceinline__ void write_row(const QueryLaunch& a, const uint64_t (
   }
 }
 
-__device__ __forceinline__ int2 load_run(const QueryLaunch& a, int row, int lane) {
-  int2 run = make_int2(0, 0);
-  if (lane < kNeighbours) run = a.runs[static_cast<int64_t>(row) * kNeighbours + lane];
+// A run from the caller's tables, emptied (and reported) when it leaves the
+// support records.
+__device__ __forceinline__ int2 checked_run(const QueryLaunch& a, int2 run) {
   if (run.y < 0 || run.x < 0 || static_cast<int64_t>(run.x) + run.y > a.n_support) {
     raise_status(&a.meta->status, kStatusTable);
     run.y = 0;
   }
   return run;
+}
+
+__device__ __forceinline__ int2 load_run(const QueryLaunch& a, int row, int lane) {
+  int2 run = make_int2(0, 0);
+  if (lane < kNeighbours) run = a.runs[static_cast<int64_t>(row) * kNeighbours + lane];
+  return checked_run(a, run);
 }
 
 // Record of query qi of a chunked item (queries q0 .. q0+qn-1 of group g0):
@@ -340,10 +488,12 @@ __device__ __noinline__ int ordered_query_row(const float4* __restrict__ qrec,
   return row;
 }
 
-// Register budget per list length (CTAs have at most 256 threads).  Without
-// one, ptxas holds the 16-entry kernels to 64 registers and spills; 96 still
-// fits the 20 resident warps per SM that the default tile's shared memory
-// allows.  Lists of up to 8 entries fit in 80 without spilling.
+// Register budget per list length (CTAs have at most 256 threads).  The
+// 16-entry kernels' 96 registers fit the 20 resident warps per SM that the
+// default tile's shared memory allows: on the 16-cloud batch (1.46 million
+// queries, K=16, whole call) 96 registers take 614 us, 80 646 us and 72
+// 686 us; lists of 8 with 80 registers (700 thousand queries) 312 us, with 64
+// 329 us; lists of 32 with 128 registers 573 us, with 96 609 us.
 template <int KCAP>
 constexpr int query_max_regs() {
   return KCAP <= 8 ? 80 : (KCAP <= 16 ? 96 : (KCAP <= 32 ? 128 : 224));
@@ -357,8 +507,7 @@ constexpr int query_max_regs() {
 template <int KCAP, bool EXACT, typename IdxT>
 __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_cands_per_lane,
                                          int q0, int qn, int g0, int k, float4* tile,
-                                         uint16_t* srt16, uint32_t* hist, uint64_t* bar,
-                                         uint32_t phase) {
+                                         uint32_t* hist, uint64_t* bar, uint32_t phase) {
   const int lane = threadIdx.x & 31;
   // One group with more candidates than a tile, up to 32 of its queries,
   // G lanes per query.  Phase A scans the first runs (the group's own
@@ -430,13 +579,16 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
         for (int t0 = 0; t0 < cnt; t0 += 32) {
           const int t = t0 + lane;
           bool keep = false;
+          float4 c = q;
           if (t < cnt) {
-            const float4 c = tile[t];
+            c = tile[t];
             const float dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
             keep = dx * dx + dy * dy + dz * dz <= rad2;
           }
+          // in place: the kept records move towards the front, never past
+          // the ones still to be read (the ballot follows every lane's read)
           const uint32_t b = __ballot_sync(kFull, keep);
-          if (keep) srt16[m + __popc(b & lanemask_lt())] = static_cast<uint16_t>(t);
+          if (keep) tile[m + __popc(b & lanemask_lt())] = c;
           m += __popc(b);
         }
         __syncwarp();
@@ -445,7 +597,7 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
       for (int i0 = 0; i0 < cnt; i0 += G) {
         const int i = i0 + sub;
         const bool ok = takes && i < cnt;
-        const float4 c = ok ? tile[filter ? srt16[i] : i] : q;
+        const float4 c = ok ? tile[i] : q;
         const float d = sq_dist(c.x, c.y, c.z, q.x, q.y, q.z);
         const uint32_t db = __float_as_uint(d);
         const bool acc = ok && db <= thr;
@@ -483,11 +635,12 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
   return static_cast<int>(phase);
 }
 
-// Shared memory of one staging buffer of a warp: the candidate tile, the
-// item's group slots and a flag word (1 = the item's groups overflowed the
+// Shared memory of one staging buffer of a warp: the candidate tile and one
+// record past it that no distance accepts (NaN coordinates), the item's group
+// slots and a flag word (1 = the item's groups overflowed the
 // tile, which only a malformed item can cause).
 __host__ __device__ constexpr size_t buffer_bytes(int T) {
-  return static_cast<size_t>(T) * 16 + kMaxGroupsPerItem * sizeof(GroupSlot) + 16;
+  return static_cast<size_t>(T) * 16 + kMaxGroupsPerItem * sizeof(GroupSlot) + 32;
 }
 
 // One warp's shared memory: `depth` staging buffers (at buf0 + b * stride)
@@ -497,16 +650,15 @@ struct WarpSmem {
   size_t stride;
   int T;
   uint64_t* bars;
-  uint16_t* tmp16;
   uint16_t* srt16;
+  uint16_t* tmp16;
   uint16_t* bstart;
-  uint8_t* qgroup;
   uint32_t* hist;
   __device__ __forceinline__ float4* tile(int b) const {
     return reinterpret_cast<float4*>(buf0 + b * stride);
   }
   __device__ __forceinline__ GroupSlot* slots(int b) const {
-    return reinterpret_cast<GroupSlot*>(buf0 + b * stride + static_cast<size_t>(T) * 16);
+    return reinterpret_cast<GroupSlot*>(buf0 + b * stride + static_cast<size_t>(T) * 16 + 16);
   }
   __device__ __forceinline__ int* flags(int b) const {
     return reinterpret_cast<int*>(slots(b) + kMaxGroupsPerItem);
@@ -521,30 +673,26 @@ __device__ __forceinline__ WarpSmem warp_smem(unsigned char* smem_raw, int T, in
   w.stride = buffer_bytes(T);
   w.T = T;
   w.bars = reinterpret_cast<uint64_t*>(smem_raw) + warp * kMaxStaging;
-  w.tmp16 = reinterpret_cast<uint16_t*>(w.buf0 + static_cast<size_t>(depth) * buffer_bytes(T));
-  w.srt16 = w.tmp16 + T;
-  w.bstart = w.srt16 + T;
-  w.qgroup = reinterpret_cast<uint8_t*>(w.bstart + kMaxGroupsPerItem * (kBuckets + 1));
-  w.hist = reinterpret_cast<uint32_t*>(w.qgroup + 32);
+  w.srt16 = reinterpret_cast<uint16_t*>(w.buf0 + static_cast<size_t>(depth) * buffer_bytes(T));
+  w.tmp16 = w.srt16 + sorted_slots(T);
+  w.bstart = w.tmp16 + T;
+  w.hist = reinterpret_cast<uint32_t*>(w.bstart + kMaxGroupsPerItem * (kBuckets + 1));
   return w;
 }
 
-__device__ __forceinline__ int pop_item(Meta* meta) {
-  int item = 0;
-  if ((threadIdx.x & 31) == 0) item = atomicAdd(&meta->queue_head, 1);
-  return __shfl_sync(kFull, item, 0);
+__device__ __forceinline__ int4 load_item(const QueryLaunch& a, int item, int n_items) {
+  return item < n_items ? a.items[item] : make_int4(0, 0, 0, 0);
 }
 
-// Checks item `item` and, for a packed item, issues the bulk copies of its
+// Checks work item `it` and, for a packed item, issues the bulk copies of its
 // groups' candidate runs into buffer b (completing on the buffer's
 // mbarrier) and records the groups in the buffer's slots.  Returns 1 when
 // copies were armed (the caller waits on the buffer's barrier), 0 for a
 // chunked item (it streams its own tiles), -1 for a malformed item (status
 // raised, nothing to do).
-__device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_groups, int T,
+__device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, int n_groups, int T,
                                           const WarpSmem& w, int b) {
   const int lane = threadIdx.x & 31;
-  const int4 it = a.items[item];
   const int q0 = it.x, qn = it.y, g0 = it.z, gn = it.w & 0xffff;
   const bool chunked = (it.w & kItemChunked) != 0;
   if (q0 < 0 || qn < 1 || qn > 32 || static_cast<int64_t>(q0) + qn > a.n_qrec || g0 < 0 ||
@@ -557,10 +705,19 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_
   if (lane < gn) {
     const int g = g0 + lane;
     const int gs = a.group_start[g], ge = a.group_start[g + 1];
+    grow = a.group_row ? a.group_row[g] : g;
     ga = max(gs, q0);
     gb = max(ga, min(ge, q0 + qn));
-    grow = a.group_row ? a.group_row[g] : g;
   }
+  // The runs of two groups ahead are in flight while a group's copies are
+  // issued.
+  auto fetch = [&](int gi) {
+    const int row = __shfl_sync(kFull, grow, gi & 31);
+    return gi < gn && lane < kNeighbours
+               ? __ldg(a.runs + static_cast<int64_t>(row) * kNeighbours + lane)
+               : make_int2(0, 0);
+  };
+  int2 run = fetch(0), run1 = fetch(1);
   __syncwarp();
   fence_proxy_async_smem();  // earlier generic accesses of the tile precede the copies
   __syncwarp();
@@ -568,12 +725,13 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_
   uint64_t* bar = w.bar(b);
   int seg = 0;
   bool overflow = false;
+#pragma unroll 1
   for (int gi = 0; gi < gn; ++gi) {
+    const int2 run2 = fetch(gi + 2);
     const int ga_ = __shfl_sync(kFull, ga, gi), gb_ = __shfl_sync(kFull, gb, gi);
-    const int row = __shfl_sync(kFull, grow, gi);
     int len = 0;
     if (gb_ > ga_ && !overflow) {
-      const int2 run = load_run(a, row, lane);
+      run = checked_run(a, run);
       const int incl = warp_inclusive_scan(run.y);
       len = __shfl_sync(kFull, incl, 31);
       if (seg + len > T) {
@@ -588,7 +746,7 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_
       }
     }
     if (lane == 0) {
-      GroupSlot s{};
+      GroupSlot s;
       s.seg = seg;
       s.len = len;
       s.a = ga_;
@@ -596,6 +754,8 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_
       w.slots(b)[gi] = s;
     }
     seg += len;
+    run = run1;
+    run1 = run2;
   }
   if (lane == 0) {
     *w.flags(b) = overflow ? 1 : 0;
@@ -605,131 +765,132 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, int item, int n_
 }
 
 // A packed item whose copies into buffer b have landed: up to 32 queries of
-// up to 16 groups, one query per lane (see the file comment).
+// up to 16 groups, one query per lane (see the file comment).  q is the
+// lane's query record; the next item is popped into `popped` before the
+// results are written.
 template <int KCAP, bool EXACT, typename IdxT>
-__device__ __forceinline__ void packed_item(const QueryLaunch& a, int item, const WarpSmem& w,
-                                            int b) {
+__device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it, const float4& q,
+                                            const WarpSmem& w, int b, bool pop, int& popped) {
   const int lane = threadIdx.x & 31;
   Meta* meta = a.meta;
-  const int4 it = a.items[item];
-  const int q0 = it.x, qn = it.y, gn = it.w & 0xffff;
+  const int qn = it.y, gn = it.w & 0xffff;
   const float4* tile = w.tile(b);
-  GroupSlot* slots = w.slots(b);
-  uint16_t* tmp16 = w.tmp16;
-  uint16_t* srt16 = w.srt16;
-  uint16_t* bstart = w.bstart;
-  uint8_t* qgroup = w.qgroup;
   uint32_t* hist = w.hist;
   const int k = a.k;
   if (*w.flags(b)) {  // the packer bounds every item by the tile; report a broken item
     if (lane == 0) raise_status(&meta->status, kStatusTable);
+    if (pop) popped = pop_item(meta);
     return;
   }
-  // query -> group map (0xff: a query no group of the item covers)
-  qgroup[lane] = 0xffu;
-  __syncwarp();
-  if (lane < gn) {
-    const GroupSlot s = slots[lane];
-    for (int p = s.a; p < s.b; ++p) qgroup[p - q0] = static_cast<uint8_t>(lane);
-  }
-  __syncwarp();
-
-  // Per group: centroid of its queries, distance buckets, counting sort.
+  // Per group: centroid of its queries, distance buckets, counting sort of
+  // its candidates' tile positions.
+  const int p = it.x + lane;
+  LaneGroup mine{0, w.srt16, w.bstart, 1.f, 0.f, 0.f};
+  bool mapped = false;
+  uint16_t* srt = w.srt16;
+#pragma unroll 1
   for (int gi = 0; gi < gn; ++gi) {
-    const GroupSlot s = slots[gi];
+    const GroupSlot s = w.slots(b)[gi];
     if (s.b <= s.a) continue;
-    const int nq = s.b - s.a;
-    float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane < nq) qv = a.qrec[s.a + lane];
-    const float inv_nq = 1.f / static_cast<float>(nq);
-    const float cx = warp_sum(qv.x) * inv_nq;
-    const float cy = warp_sum(qv.y) * inv_nq;
-    const float cz = warp_sum(qv.z) * inv_nq;
-    float d2max = 0.f;
-    for (int t = lane; t < s.len; t += 32) {
-      const float4 c = tile[s.seg + t];
-      const float dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
-      d2max = fmaxf(d2max, dx * dx + dy * dy + dz * dz);
+    const bool member = p >= s.a && p < s.b;  // a subset of the item's qn lanes
+    const float inv_nq = 1.f / static_cast<float>(s.b - s.a);
+    const float cx = warp_sum(member ? q.x : 0.f) * inv_nq;
+    const float cy = warp_sum(member ? q.y : 0.f) * inv_nq;
+    const float cz = warp_sum(member ? q.z : 0.f) * inv_nq;
+    const float4* seg = tile + s.seg;
+    // The buckets' range: the largest squared distance to the centroid among
+    // 32 evenly spaced candidates (the last bucket takes all beyond).
+    float far2 = 0.f;
+    if (s.len > 0) {
+      const float4 c = seg[(lane * s.len) >> 5];
+      far2 = fmaxf(far2, sq_dist(c.x, c.y, c.z, cx, cy, cz));
     }
-    d2max = warp_max(d2max);
-    const float w2 = d2max > 0.f ? d2max * (1.0f / kBuckets) * 1.0001f : 1.f;
+    far2 = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(far2)));
+    const float w2 = far2 > 0.f ? far2 * (1.0f / kBuckets) * 1.0001f : 1.f;
     const float inv_w2 = 1.f / w2;
     hist[lane] = 0u;  // kBuckets == 32: one bucket per lane
     __syncwarp();
     // Bucket of every candidate and its rank inside the bucket.
+#pragma unroll 2
     for (int t = lane; t < s.len; t += 32) {
-      const float4 c = tile[s.seg + t];
-      const float dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
-      const int bkt = min(static_cast<int>((dx * dx + dy * dy + dz * dz) * inv_w2), kBuckets - 1);
+      const float4 c = seg[t];
+      const float d2 = sq_dist(c.x, c.y, c.z, cx, cy, cz);
+      const int bkt = min(static_cast<int>(d2 * inv_w2), kBuckets - 1);
       const uint32_t r = atomicAdd(&hist[bkt], 1u);
-      tmp16[s.seg + t] = static_cast<uint16_t>((bkt << 10) | r);
+      w.tmp16[t] = static_cast<uint16_t>((bkt << 10) | r);
     }
     __syncwarp();
     const uint32_t h = hist[lane];
     const uint32_t hi = static_cast<uint32_t>(warp_inclusive_scan(static_cast<int>(h)));
-    uint16_t* bs = bstart + gi * (kBuckets + 1);
+    uint16_t* bs = w.bstart + gi * (kBuckets + 1);
     bs[lane] = static_cast<uint16_t>(hi - h);
     if (lane == 31) bs[kBuckets] = static_cast<uint16_t>(hi);
     __syncwarp();
-    hist[lane] = hi - h;
-    __syncwarp();
+#pragma unroll 2
     for (int t = lane; t < s.len; t += 32) {
-      const uint16_t v = tmp16[s.seg + t];
-      const int bkt = v >> 10;
-      srt16[s.seg + hist[bkt] + (v & 1023)] = static_cast<uint16_t>(s.seg + t);
+      const uint32_t v = w.tmp16[t];
+      srt[bs[v >> 10] + (v & 1023u)] = static_cast<uint16_t>(s.seg + t);
     }
-    if (lane == 0) {
-      const float mag = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + sqrtf(d2max);
-      slots[gi].cx = cx;
-      slots[gi].cy = cy;
-      slots[gi].cz = cz;
-      slots[gi].inv_w2 = inv_w2;
-      slots[gi].eps = mag * 4e-6f + 1e-30f;
+    if (lane < ((-s.len) & 7)) srt[s.len + lane] = static_cast<uint16_t>(w.T);  // no candidate
+    if (member) {
+      const float dx = q.x - cx, dy = q.y - cy, dz = q.z - cz;
+      const float mag = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + sqrtf(far2);
+      mapped = true;
+      mine.len = cut_accepts_any(a.cut_r2) ? s.len : 0;
+      mine.srt = srt;
+      mine.bstart = bs;
+      mine.inv_w2 = inv_w2;
+      mine.rq = sqrtf(dx * dx + dy * dy + dz * dz);
+      mine.eps = mag * 4e-6f + 1e-30f;
     }
+    srt += (s.len + 7) & ~7;
     __syncwarp();
   }
 
   // One query per lane.
-  const int mapped = lane < qn ? qgroup[lane] : 0;
-  if (lane < qn && mapped >= gn) raise_status(&meta->status, kStatusTable);
-  const bool active = lane < qn && mapped < gn;
-  const int gi = active ? mapped : 0;
-  const GroupSlot s = slots[gi];
-  const uint16_t* bs = bstart + gi * (kBuckets + 1);
-  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (active) q = a.qrec[q0 + lane];
-  const float rdx = q.x - s.cx, rdy = q.y - s.cy, rdz = q.z - s.cz;
-  const float rq = sqrtf(rdx * rdx + rdy * rdy + rdz * rdz);
-  const int len = active && cut_accepts_any(a.cut_r2) ? s.len : 0;
+  if (lane < qn && !mapped) raise_status(&meta->status, kStatusTable);
   const uint32_t cut_lim = cut_limit(a.cut_r2);
-
-  uint64_t L[KCAP];
-#pragma unroll
-  for (int j = 0; j < KCAP; ++j) {
-    uint64_t key = kEmpty;
-    if (j < len) {
-      const float4 c = tile[srt16[s.seg + j]];
-      const float d = sq_dist(c.x, c.y, c.z, q.x, q.y, q.z);
-      if (__float_as_uint(d) <= cut_lim) key = make_key(d, c.w);
-    }
-    L[j] = key;
-  }
-  sort_network<KCAP, 0, KCAP>(L);
-  uint32_t thr = kth_limit(L[KCAP - 1], cut_lim);
-  int stop = len > 0 ? stop_position<KCAP>(L, s, rq, bs) : 0;
-  // Candidate t of the lane's scan: accepted when it beats the K-th.
-  auto test = [&](int t, uint64_t& x) {
-    const float4 c = tile[srt16[s.seg + t]];
-    const float d = sq_dist(c.x, c.y, c.z, q.x, q.y, q.z);
-    const bool acc = __float_as_uint(d) <= thr;
-    if (acc) x = make_key(d, c.w);
-    return acc;
+  // Squared distance bits of the candidate at tile position pos.
+  auto dist_bits = [&](uint32_t pos, float4& c) {
+    c = tile[pos];
+    return __float_as_uint(sq_dist(c.x, c.y, c.z, q.x, q.y, q.z));
   };
-  if constexpr (KCAP <= 16) {
+  uint64_t L[KCAP];
+  if constexpr (KCAP >= 8) {
+    select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, meta, pop,
+                        popped);
+  } else {
+    const int len = mine.len;
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j) {
+      uint64_t key = kEmpty;
+      if (j < len) {
+        float4 c;
+        const uint32_t d = dist_bits(mine.srt[j], c);
+        if (d <= cut_lim) key = make_key(__uint_as_float(d), c.w);
+      }
+      L[j] = key;
+    }
+    sort_network<KCAP, 0, KCAP>(L);
+    uint32_t thr = kth_limit(L[KCAP - 1], cut_lim);
+    auto kth_stop = [&] {
+      const uint64_t last = L[KCAP - 1];
+      return last == kEmpty
+                 ? len
+                 : stop_position(__uint_as_float(static_cast<uint32_t>(last >> 32)), mine);
+    };
+    int stop = len > 0 ? kth_stop() : 0;
+    // Candidate t of the lane's scan: accepted when it beats the K-th.
+    auto test = [&](int t, uint64_t& x) {
+      float4 c;
+      const uint32_t d = dist_bits(mine.srt[t], c);
+      const bool acc = d <= thr;
+      if (acc) x = make_key(__uint_as_float(d), c.w);
+      return acc;
+    };
     // Two candidates per iteration, both tested against the same K-th
     // distance: half the loop and vote overhead, and two independent loads
-    // and distance chains in flight.  (With a 32- or 64-entry list the
-    // extra registers cost more than this saves.)
+    // and distance chains in flight.
     for (int t = KCAP;; t += 2) {
       const bool live0 = t < stop, live1 = t + 1 < stop;
       if (!__any_sync(kFull, live0)) break;
@@ -745,29 +906,16 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, int item, cons
       }
       const bool any0 = __any_sync(kFull, acc0 || acc1);
       const bool any1 = __any_sync(kFull, acc0 && acc1);
-      if (any0) insert_one<KCAP>(L, x0);
-      if (any1) insert_one<KCAP>(L, x1);
+      if (any0) list_insert<KCAP>(L, x0);
+      if (any1) list_insert<KCAP>(L, x1);
       if (acc0 || acc1) {
         thr = kth_limit(L[KCAP - 1], cut_lim);
-        stop = min(stop, stop_position<KCAP>(L, s, rq, bs));
+        stop = min(stop, kth_stop());
       }
     }
-  } else {
-    for (int t = KCAP;; ++t) {
-      const bool live = t < stop;
-      if (!__any_sync(kFull, live)) break;
-      uint64_t x = kEmpty;
-      const bool acc = live && test(t, x);
-      if (__any_sync(kFull, acc)) {
-        insert_one<KCAP>(L, x);
-        if (acc) {
-          thr = kth_limit(L[KCAP - 1], cut_lim);
-          stop = min(stop, stop_position<KCAP>(L, s, rq, bs));
-        }
-      }
-    }
+    if (pop) popped = pop_item(meta);
   }
-  if (active) write_row<IdxT, KCAP, EXACT>(a, L, __float_as_int(q.w), k);
+  if (lane < qn && mapped) write_row<IdxT, KCAP, EXACT>(a, L, __float_as_int(q.w), k);
   __syncwarp();
 }
 
@@ -800,7 +948,11 @@ __global__ void __maxnreg__(query_max_regs<KCAP>())
   const WarpSmem w = warp_smem(smem_raw, T, depth);
   Meta* meta = a.meta;
   if (lane == 0) {
-    for (int b = 0; b < depth; ++b) mbar_init(w.bar(b), 1);
+    const float nan = __int_as_float(0x7fffffff);
+    for (int b = 0; b < depth; ++b) {
+      mbar_init(w.bar(b), 1);
+      w.tile(b)[T] = make_float4(nan, nan, nan, 0.f);
+    }
     mbar_init_fence();
   }
   __syncwarp();
@@ -810,43 +962,52 @@ __global__ void __maxnreg__(query_max_regs<KCAP>())
   const int n_groups = *a.group_count_ptr;
 
   int buf = 0;
-  int item = pop_item(meta);
-  int staged = item < n_items ? stage_item(a, item, n_groups, T, w, buf) : -1;
+  int item = item_of(pop_item(meta));
+  int4 it = load_item(a, item, n_items);
+  int staged = item < n_items ? stage_item(a, it, n_groups, T, w, buf) : -1;
   if (staged == 1) pending |= 1u << buf;
   while (item < n_items) {
-    int next = n_items, next_staged = -1;
+    int popped = 0, next = n_items, next_staged = -1;
+    int4 next_it = make_int4(0, 0, 0, 0);
     if (depth > 1) {  // the next item's copies fly while this one is scanned
-      next = pop_item(meta);
-      if (next < n_items) next_staged = stage_item(a, next, n_groups, T, w, buf ^ 1);
+      next = item_of(pop_item(meta));
+      next_it = load_item(a, next, n_items);
+      if (next < n_items) next_staged = stage_item(a, next_it, n_groups, T, w, buf ^ 1);
       if (next_staged == 1) pending |= 1u << (buf ^ 1);
     }
     if (staged == 1) {
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (lane < it.y) q = a.qrec[it.x + lane];  // in flight during the wait
       if (!mbar_wait_bounded(w.bar(buf), (phase >> buf) & 1u, kWaitLimit)) {
         drain_after_timeout(meta, w, phase, pending, depth);
         return;
       }
       phase ^= 1u << buf;
       pending &= ~(1u << buf);
-      packed_item<KCAP, EXACT, IdxT>(a, item, w, buf);
-    } else if (staged == 0) {
-      const int4 it = a.items[item];
-      const int nxt = chunked_item<KCAP, EXACT, IdxT>(a, T, min_cands_per_lane, it.x, it.y, it.z,
-                                                      a.k, w.tile(buf), w.srt16, w.hist,
-                                                      w.bar(buf), (phase >> buf) & 1u);
-      if (nxt < 0) {  // its own copies were waited for; the other buffer's may fly
-        drain_after_timeout(meta, w, phase, pending, depth);
-        return;
+      packed_item<KCAP, EXACT, IdxT>(a, it, q, w, buf, depth == 1, popped);
+    } else {
+      if (staged == 0) {
+        const int nxt = chunked_item<KCAP, EXACT, IdxT>(a, T, min_cands_per_lane, it.x, it.y, it.z,
+                                                        a.k, w.tile(buf), w.hist, w.bar(buf),
+                                                        (phase >> buf) & 1u);
+        if (nxt < 0) {  // its own copies were waited for; the other buffer's may fly
+          drain_after_timeout(meta, w, phase, pending, depth);
+          return;
+        }
+        phase = (phase & ~(1u << buf)) | (static_cast<uint32_t>(nxt) << buf);
       }
-      phase = (phase & ~(1u << buf)) | (static_cast<uint32_t>(nxt) << buf);
+      if (depth == 1) popped = pop_item(meta);
     }
     if (depth > 1) {
       buf ^= 1;
     } else {
-      next = pop_item(meta);
-      if (next < n_items) next_staged = stage_item(a, next, n_groups, T, w, buf);
+      next = item_of(popped);
+      next_it = load_item(a, next, n_items);
+      if (next < n_items) next_staged = stage_item(a, next_it, n_groups, T, w, buf);
       if (next_staged == 1) pending |= 1u << buf;
     }
     item = next;
+    it = next_it;
     staged = next_staged;
   }
   __syncwarp();

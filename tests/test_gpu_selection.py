@@ -1,0 +1,66 @@
+"""The packed scan's 32-bit block selection where it can go wrong: distances
+that differ only in the bits its keys drop, exact ties at the K-th place,
+candidate counts around the block size, K below the list's capacity, both
+position widths -- bit-exact against the oracle."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _check(xyz, k, voxel, config=None, cut_r2=math.inf):
+    import flashknn_exprepo_b200 as fk
+    offs = np.array([len(xyz)])
+    oi, od = O.knn_offsets(xyz, offs, k, voxel, 2, cut_r2=np.float32(cut_r2))
+    gi, gd = fk.ops.knn_offsets(torch.from_numpy(xyz).to(DEV), torch.from_numpy(offs).to(DEV), k,
+                                voxel, 2, cut_r2=cut_r2, config=config, validate=True)
+    assert np.array_equal(gi.cpu().numpy(), oi)
+    assert np.array_equal(gd.cpu().numpy().view(np.uint32), od.view(np.uint32))
+
+
+def _lattice(side, jitter):
+    """A shuffled unit lattice, every coordinate moved by up to `jitter`: the
+    neighbours' distances fall into a few classes, equal (jitter 0) or apart
+    by less than the keys resolve."""
+    rng = np.random.default_rng(side)
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    xyz = g.astype(np.float32) + np.float32(0.5)
+    xyz = xyz + (rng.random(xyz.shape, dtype=np.float32) - np.float32(0.5)) * np.float32(2 * jitter)
+    rng.shuffle(xyz)
+    return np.ascontiguousarray(xyz, dtype=np.float32)
+
+
+@pytest.mark.parametrize("jitter", [0.0, 2e-6, 2e-5, 1e-3])
+@pytest.mark.parametrize("k", [5, 8, 9, 16, 17, 24, 32, 33, 64])
+def test_distance_classes(k, jitter):
+    _check(_lattice(17, jitter), k, 0.5)
+
+
+@pytest.mark.parametrize("k", [8, 16, 32])
+def test_wide_tile_positions(k):
+    from flashknn_exprepo_b200 import _lib
+    xyz = _lattice(17, 2e-5)
+    for voxel in (0.5, 0.7):  # 216 and up to 729 candidates per cell neighbourhood
+        _check(xyz, k, voxel, _lib.FknnConfig(2, 1024, 8, 0, 1))
+        _check(xyz, k, voxel, _lib.FknnConfig(2, 512, 8, 0, 2))
+
+
+@pytest.mark.parametrize("k", [5, 8, 16, 24])
+def test_candidate_counts_around_a_block(k):
+    """Cells far apart, each its own neighbourhood of 1..70 points, some of
+    them duplicates."""
+    rng = np.random.default_rng(k)
+    parts = [rng.random((n, 3), dtype=np.float32) * np.float32(0.3) + np.float32(4 * n)
+             for n in range(1, 71)]
+    xyz = np.concatenate(parts)
+    dup = rng.integers(0, len(xyz), len(xyz) // 4)
+    xyz = np.ascontiguousarray(np.concatenate([xyz, xyz[dup]]))
+    _check(xyz, k, 0.1)
+    _check(xyz, k, 0.1, cut_r2=0.01)
