@@ -147,6 +147,23 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
+// ------------------------------------------------------- 16-byte copies
+// Asynchronous copy global -> shared memory of 16 aligned bytes; the thread
+// commits its copies as a group and waits until at most N groups are pending.
+__device__ __forceinline__ void copy_16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void copy_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // ------------------------------------------------------ warp primitives
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;

@@ -12,17 +12,19 @@
 //     (atomicAdd on Meta::queue_head);
 //   * packed item: up to 32 consecutive queries from up to 32 consecutive
 //     groups, one query per lane.  Each group's 27 runs are staged into the
-//     warp's shared-memory tile by non-multicast cp.async.bulk copies that
-//     complete on the warp's mbarrier.  Each group's candidates are then
+//     warp's shared-memory tile, one 16-byte cp.async per record (the runs
+//     are short: a bulk copy each, issued lane after lane, took longer).
+//     Each group's candidates are then
 //     counting-sorted (32 buckets of squared distance) by distance to the
-//     centroid of the group's queries, so every lane meets near candidates
+//     centre of the group's queries, so every lane meets near candidates
 //     first and stops at the first bucket whose lower distance bound exceeds
 //     its current K-th distance (triangle inequality, with a safety margin
 //     for FP32 rounding).  Lists of 8 and more take the candidates in blocks
 //     sorted and merged as 32-bit keys (select_blocks); shorter ones insert
 //     them one by one when some lane improves (warp vote);
 //   * chunked item: one group with more candidates than a tile; G lanes per
-//     query split its candidates, streamed tile by tile, and the G partial
+//     query split its candidates, streamed tile by tile by non-multicast
+//     cp.async.bulk copies on the warp's mbarrier, and the G partial
 //     lists are merged with xor-shuffle bitonic merges;
 //   * results come from packed u64 keys (distance bits << 32 | index), so
 //     ordering is exact including ties; rows are written straight to the caller's
@@ -58,7 +60,7 @@ struct LaneGroup {
   const uint16_t* srt;       // their tile positions in bucket order
   const uint16_t* bstart;    // first of every bucket
   float inv_w2;              // 1 / bucket width in squared distance
-  float rq;                  // distance of the query to the group's centroid
+  float rq;                  // distance of the query to the group's centre (a little above)
   float eps;                 // absolute margin of the early-exit bound
 };
 
@@ -197,52 +199,81 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Warp-wide minimum / maximum of a float in one instruction (NaN: ignored).
+__device__ __forceinline__ float redux_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+__device__ __forceinline__ float redux_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, s));
   return v;
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_addr(bar))
-      : "memory");
+// A little above sqrt(d): d * rsqrt(d) is within a few ulp of it, far inside
+// the 1e-4 margin.  d >= FLT_MIN keeps a distance of 0 (a query on a support
+// point) or a subnormal one bounded from above, and +inf gives NaN, which
+// skips no bucket.
+__device__ __forceinline__ float sqrt_above(float d) {
+  const float m = fmaxf(d, FLT_MIN);
+  return m * rsqrtf(m) * 1.0001f;
 }
 
 // First sorted position whose bucket cannot hold a candidate closer than the
-// lane's current KCAP-th distance.  Buckets are uniform in the squared
-// distance to the centroid: a candidate in bucket b lies at least
-// sqrt(b*w2) from the centroid, hence at least sqrt(b*w2) - rq from the
+// lane's current K-th distance `kth`.  Buckets are uniform in the squared
+// distance to the group's centre: a candidate in bucket b lies at least
+// sqrt(b*w2) from the centre, hence at least sqrt(b*w2) - rq from the
 // query; buckets with b*w2 > (rq + sqrt(thr))^2 (plus margins) are skipped.
 __device__ __forceinline__ int stop_position(float kth, const LaneGroup& s) {
-  // m * rsqrt(m) is within a few ulp of sqrt(m), far inside the 1e-4 margin;
-  // m >= FLT_MIN keeps a K-th distance of 0 (a query on a support point) or
-  // a subnormal one bounded from above, and +inf gives NaN, which skips no
-  // bucket
-  const float m = fmaxf(kth, FLT_MIN);
-  const float reach = s.rq + m * rsqrtf(m) * 1.0001f + s.eps;
+  const float reach = s.rq + sqrt_above(kth) + s.eps;
   const float lim = reach * reach * s.inv_w2;
   if (!(lim < static_cast<float>(kBuckets - 1))) return s.len;
   return s.bstart[static_cast<int>(lim) + 1];
 }
 
-// The next item of the queue, in lane 0 (item_of() gives it to every lane),
-// so that the atomic is in flight while the warp finishes its current item.
-__device__ __forceinline__ int pop_item(Meta* meta) {
-  return (threadIdx.x & 31) == 0 ? atomicAdd(&meta->queue_head, 1) : 0;
-}
-__device__ __forceinline__ int item_of(int popped) { return __shfl_sync(kFull, popped, 0); }
+// The work item a warp takes next, fetched while it finishes the current one:
+// the queue's atomic, then the item's descriptor, are in flight meanwhile.
+// The pop comes late in an item, so that a warp never holds an item it is far
+// from starting while others run out.
+struct NextItem {
+  bool wanted;  // false: the item is taken elsewhere (staging depth 2)
+  int popped;   // lane 0
+  int item;
+  int4 it;
+  int gs, ge, row;  // lane's group: query range and runs row (garbage past the item's groups)
+  __device__ __forceinline__ void pop(Meta* meta) {
+    if (wanted && (threadIdx.x & 31) == 0) popped = atomicAdd(&meta->queue_head, 1);
+  }
+  __device__ __forceinline__ void load(const QueryLaunch& a, int n_items) {
+    if (!wanted) return;
+    item = __shfl_sync(kFull, popped, 0);
+    if (item < n_items) it = a.items[item];
+  }
+  // The groups of a well-formed item, one per lane (stage_item checks it).
+  __device__ __forceinline__ void load_groups(const QueryLaunch& a, int n_items, int n_groups) {
+    if (!wanted || item >= n_items) return;
+    const int lane = threadIdx.x & 31;
+    const int g = it.z + lane;
+    if (it.z >= 0 && it.z < n_groups && lane < (it.w & 0xffff) && g < n_groups) {
+      gs = a.group_start[g];
+      ge = a.group_start[g + 1];
+      row = a.group_row ? a.group_row[g] : g;
+    }
+  }
+};
 
 // Order-preserving 32-bit keys of the packed scan: the squared distance's
-// bits with the low ones replaced by the candidate's position in its group's
-// sorted list, so a compare-exchange is a min and a max.
+// bits with the low ones replaced by the candidate's tile position, so a compare-exchange is a min and a max.
 constexpr uint32_t kNone32 = ~0u;
+constexpr uint32_t kInfBits = 0x7f800000u;
 
 // Merges the ascending block X into the ascending list L, keeping the KCAP
 // smallest; dropped = the smallest key ever left out.
@@ -270,14 +301,14 @@ __device__ __forceinline__ void merge_block(uint32_t (&L)[KCAP], const uint32_t 
 // Bound by instruction issue.  The scan sorts blocks of B candidates as
 // 32-bit keys and merges each block into the list (a minimum and a maximum
 // per compare-exchange), in place of one warp-wide 64-bit insertion per
-// accepted candidate of any lane: 309 -> about 200 warp instructions per
-// query at K=16.  The first block goes through the same loop as the rest (no
+// accepted candidate of any lane: 309 -> 190 warp instructions per query at
+// K=16.  The first block goes through the same loop as the rest (no
 // separate fill): the code the warps share has to stay small, since straight
 // copies of it made instruction fetch the first stall (2.8 of 10 cycles per
-// instruction).  With the sort's reworked loops the whole call over the
-// 16-cloud batch (1.46 million queries, K=16) went from 861 to 614 us, over
-// 700 thousand queries at K=32 from 880 to 573 us, over 300 thousand at K=64
-// from 1182 to 607 us.  The keys
+// instruction).  With staging and sort the whole call over the 16-cloud batch
+// (1.46 million queries, K=16) went from 861 to 574 us, over 700 thousand
+// queries at K=32 from 880 to 484 us, over 300 thousand at K=64 from 1182 to
+// 522 us.  The keys
 // drop the low 9 or 10 bits of the distance, so the exact keys of the list
 // are computed at the end and neighbours that the truncation left in the
 // wrong order are exchanged; a lane whose k-th entry shares its truncated
@@ -286,30 +317,28 @@ __device__ __forceinline__ void merge_block(uint32_t (&L)[KCAP], const uint32_t 
 template <int KCAP, typename DistBits>
 __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGroup& g, int k,
                                               uint32_t pos_mask, uint32_t cut_lim,
-                                              DistBits& dist_bits, Meta* meta, bool pop,
-                                              int& popped) {
+                                              DistBits& dist_bits, const QueryLaunch& a,
+                                              int n_items, uint32_t none, NextItem& next) {
   constexpr int B = KCAP <= 16 ? 8 : 16;
   const uint16_t* srt = g.srt;
   uint32_t L[KCAP];
   uint32_t dropped = kNone32, last = kNone32;
 #pragma unroll
   for (int j = 0; j < KCAP; ++j) L[j] = kNone32;
-  int stop = g.len;
+  int stop = min(g.len, stop_position(__uint_as_float(cut_lim), g));
 #pragma unroll 1
   for (int t0 = 0; __any_sync(kFull, t0 < stop); t0 += B) {
     uint32_t X[B];
 #pragma unroll
     for (int h = 0; h < B; h += 8) {  // eight positions per 16-byte load
-      const bool live = t0 + h < stop;
-      uint4 p = make_uint4(0u, 0u, 0u, 0u);
-      if (live) p = *reinterpret_cast<const uint4*>(srt + t0 + h);
+      uint4 p = make_uint4(none, none, none, none);
+      if (t0 + h < stop) p = *reinterpret_cast<const uint4*>(srt + t0 + h);
       const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         float4 c;
-        const uint32_t d = dist_bits((u & 1) ? pw[u >> 1] >> 16 : pw[u >> 1] & 0xffffu, c);
-        X[h + u] = live && d <= cut_lim ? (d & ~pos_mask) | static_cast<uint32_t>(t0 + h + u)
-                                        : kNone32;
+        const uint32_t pos = (u & 1) ? pw[u >> 1] >> 16 : pw[u >> 1] & 0xffffu;
+        X[h + u] = (dist_bits(pos, c) & ~pos_mask) | pos;
       }
     }
     sort_network<B, 0, B>(X);
@@ -321,24 +350,28 @@ __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGro
         for (int j = 0; j < KCAP - 1; ++j)
           if (j == k - 1) last = L[j];
       }
-      if (last != kNone32) stop = min(stop, stop_position(__uint_as_float(last | pos_mask), g));
+      stop = min(stop, stop_position(__uint_as_float(min(last | pos_mask, cut_lim)), g));
     } else {
       dropped = min(dropped, X[0]);
     }
   }
-  if (pop) popped = pop_item(meta);
-  // Exact keys; entries of an ambiguous k-th truncated distance stay out.
-  const bool ambiguous = last != kNone32 && ((dropped ^ last) & ~pos_mask) == 0u;
-  const uint32_t limit = ambiguous ? last & ~pos_mask : kNone32;
+  next.pop(a.meta);
+  // Exact keys.  Candidates outside the cut (NaN: no candidate) went through
+  // the list like the others, behind every one inside; they end here, and so
+  // do the entries of an ambiguous k-th truncated distance.
+  const bool ambiguous =
+      (last & ~pos_mask) <= cut_lim && ((dropped ^ last) & ~pos_mask) == 0u;
+  const uint32_t limit = ambiguous ? last & ~pos_mask : kInfBits;
 #pragma unroll
   for (int j = 0; j < KCAP; ++j) {
     E[j] = kEmpty;
     if (L[j] < limit) {
       float4 c;
-      const uint32_t d = dist_bits(srt[L[j] & pos_mask], c);
-      E[j] = make_key(__uint_as_float(d), c.w);
+      const uint32_t d = dist_bits(L[j] & pos_mask, c);
+      if (d <= cut_lim) E[j] = make_key(__uint_as_float(d), c.w);
     }
   }
+  next.load(a, n_items);
   while (true) {
     bool sorted = true;
 #pragma unroll
@@ -491,9 +524,9 @@ __device__ __noinline__ int ordered_query_row(const float4* __restrict__ qrec,
 // Register budget per list length (CTAs have at most 256 threads).  The
 // 16-entry kernels' 96 registers fit the 20 resident warps per SM that the
 // default tile's shared memory allows: on the 16-cloud batch (1.46 million
-// queries, K=16, whole call) 96 registers take 614 us, 80 646 us and 72
-// 686 us; lists of 8 with 80 registers (700 thousand queries) 312 us, with 64
-// 329 us; lists of 32 with 128 registers 573 us, with 96 609 us.
+// queries, K=16, whole call) 80 registers took 5 % longer and 72 12 %; lists
+// of 8 (700 thousand queries) with 64 registers instead of 80 5 %; lists of
+// 32 with 112 instead of 128 7 %, with 120 4 %.
 template <int KCAP>
 constexpr int query_max_regs() {
   return KCAP <= 8 ? 80 : (KCAP <= 16 ? 96 : (KCAP <= 32 ? 128 : 224));
@@ -680,19 +713,15 @@ __device__ __forceinline__ WarpSmem warp_smem(unsigned char* smem_raw, int T, in
   return w;
 }
 
-__device__ __forceinline__ int4 load_item(const QueryLaunch& a, int item, int n_items) {
-  return item < n_items ? a.items[item] : make_int4(0, 0, 0, 0);
-}
-
-// Checks work item `it` and, for a packed item, issues the bulk copies of its
-// groups' candidate runs into buffer b (completing on the buffer's
-// mbarrier) and records the groups in the buffer's slots.  Returns 1 when
-// copies were armed (the caller waits on the buffer's barrier), 0 for a
-// chunked item (it streams its own tiles), -1 for a malformed item (status
-// raised, nothing to do).
-__device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, int n_groups, int T,
+// Checks work item `it` and, for a packed item, issues the copies of its
+// groups' candidate runs into buffer b (the caller commits and waits for
+// them) and records the groups in the buffer's slots.  Returns 1 when copies
+// were issued, 0 for a chunked item (it streams its own tiles), -1 for a
+// malformed item (status raised, nothing to do).
+__device__ __forceinline__ int stage_item(const QueryLaunch& a, const NextItem& x, int n_groups, int T,
                                           const WarpSmem& w, int b) {
   const int lane = threadIdx.x & 31;
+  const int4 it = x.it;
   const int q0 = it.x, qn = it.y, g0 = it.z, gn = it.w & 0xffff;
   const bool chunked = (it.w & kItemChunked) != 0;
   if (q0 < 0 || qn < 1 || qn > 32 || static_cast<int64_t>(q0) + qn > a.n_qrec || g0 < 0 ||
@@ -703,11 +732,9 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, 
   if (chunked) return 0;
   int ga = 0, gb = 0, grow = 0;
   if (lane < gn) {
-    const int g = g0 + lane;
-    const int gs = a.group_start[g], ge = a.group_start[g + 1];
-    grow = a.group_row ? a.group_row[g] : g;
-    ga = max(gs, q0);
-    gb = max(ga, min(ge, q0 + qn));
+    grow = x.row;
+    ga = max(x.gs, q0);
+    gb = max(ga, min(x.ge, q0 + qn));
   }
   // The runs of two groups ahead are in flight while a group's copies are
   // issued.
@@ -718,11 +745,8 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, 
                : make_int2(0, 0);
   };
   int2 run = fetch(0), run1 = fetch(1);
-  __syncwarp();
-  fence_proxy_async_smem();  // earlier generic accesses of the tile precede the copies
-  __syncwarp();
   float4* tile = w.tile(b);
-  uint64_t* bar = w.bar(b);
+  int* base = reinterpret_cast<int*>(w.hist);  // one per non-empty run
   int seg = 0;
   bool overflow = false;
 #pragma unroll 1
@@ -733,16 +757,29 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, 
     if (gb_ > ga_ && !overflow) {
       run = checked_run(a, run);
       const int incl = warp_inclusive_scan(run.y);
+      const int first = incl - run.y;
       len = __shfl_sync(kFull, incl, 31);
       if (seg + len > T) {
         overflow = true;
         len = 0;
-      } else if (len > 0) {
-        if (lane == 0) mbar_expect_tx(bar, static_cast<uint32_t>(len) * 16u);
+      } else {
+        const uint32_t filled = __ballot_sync(kFull, run.y > 0);
+        if (run.y > 0) base[__popc(filled & lanemask_lt())] = run.x - first;
         __syncwarp();
-        if (run.y > 0)
-          bulk_copy_g2s(tile + seg + (incl - run.y), a.srec + run.x,
-                        static_cast<uint32_t>(run.y) * 16u, bar);
+        // 32 records a step, one per lane: a lane's run is the last one that
+        // starts at or before its record
+        int before = -1;
+#pragma unroll 1
+        for (int t0 = 0; t0 < len; t0 += 32) {
+          const int at = first - t0;
+          const uint32_t starts =
+              __reduce_or_sync(kFull, run.y > 0 && at >= 0 && at < 32 ? 1u << at : 0u);
+          const int r = before + __popc(starts & (lanemask_lt() | (1u << lane)));
+          before += __popc(starts);
+          if (t0 + lane < len)
+            copy_16_async(tile + seg + t0 + lane, a.srec + (base[r] + t0 + lane));
+        }
+        __syncwarp();
       }
     }
     if (lane == 0) {
@@ -757,20 +794,18 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, const int4& it, 
     run = run1;
     run1 = run2;
   }
-  if (lane == 0) {
-    *w.flags(b) = overflow ? 1 : 0;
-    mbar_arrive(bar);
-  }
+  if (lane == 0) *w.flags(b) = overflow ? 1 : 0;
   return 1;
 }
 
 // A packed item whose copies into buffer b have landed: up to 32 queries of
 // up to 16 groups, one query per lane (see the file comment).  q is the
-// lane's query record; the next item is popped into `popped` before the
-// results are written.
+// lane's query record; the next item is fetched before the results are
+// written.
 template <int KCAP, bool EXACT, typename IdxT>
 __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it, const float4& q,
-                                            const WarpSmem& w, int b, bool pop, int& popped) {
+                                            const WarpSmem& w, int b, int n_items,
+                                            int n_groups, NextItem& next) {
   const int lane = threadIdx.x & 31;
   Meta* meta = a.meta;
   const int qn = it.y, gn = it.w & 0xffff;
@@ -779,11 +814,16 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
   const int k = a.k;
   if (*w.flags(b)) {  // the packer bounds every item by the tile; report a broken item
     if (lane == 0) raise_status(&meta->status, kStatusTable);
-    if (pop) popped = pop_item(meta);
+    next.pop(meta);
+    next.load(a, n_items);
+    next.load_groups(a, n_items, n_groups);
     return;
   }
-  // Per group: centroid of its queries, distance buckets, counting sort of
-  // its candidates' tile positions.
+  // Per group: centre of its queries' box, distance buckets, counting sort of
+  // its candidates' tile positions.  Kept short rather than unrolled, with
+  // the box from six reductions instead of a centroid from fifteen shuffles:
+  // unrolled by two or four the whole call at K=32 took 533 / 552 us, as here
+  // 510 us (700 thousand queries).
   const int p = it.x + lane;
   LaneGroup mine{0, w.srt16, w.bstart, 1.f, 0.f, 0.f};
   bool mapped = false;
@@ -793,12 +833,12 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
     const GroupSlot s = w.slots(b)[gi];
     if (s.b <= s.a) continue;
     const bool member = p >= s.a && p < s.b;  // a subset of the item's qn lanes
-    const float inv_nq = 1.f / static_cast<float>(s.b - s.a);
-    const float cx = warp_sum(member ? q.x : 0.f) * inv_nq;
-    const float cy = warp_sum(member ? q.y : 0.f) * inv_nq;
-    const float cz = warp_sum(member ? q.z : 0.f) * inv_nq;
+    const float inf = __int_as_float(kInfBits);
+    const float cx = 0.5f * (redux_min(member ? q.x : inf) + redux_max(member ? q.x : -inf));
+    const float cy = 0.5f * (redux_min(member ? q.y : inf) + redux_max(member ? q.y : -inf));
+    const float cz = 0.5f * (redux_min(member ? q.z : inf) + redux_max(member ? q.z : -inf));
     const float4* seg = tile + s.seg;
-    // The buckets' range: the largest squared distance to the centroid among
+    // The buckets' range: the largest squared distance to the centre among
     // 32 evenly spaced candidates (the last bucket takes all beyond).
     float far2 = 0.f;
     if (s.len > 0) {
@@ -806,12 +846,11 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
       far2 = fmaxf(far2, sq_dist(c.x, c.y, c.z, cx, cy, cz));
     }
     far2 = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(far2)));
-    const float w2 = far2 > 0.f ? far2 * (1.0f / kBuckets) * 1.0001f : 1.f;
-    const float inv_w2 = 1.f / w2;
+    const float inv_w2 = far2 > 0.f ? __fdividef(kBuckets / 1.0001f, far2) : 1.f;
     hist[lane] = 0u;  // kBuckets == 32: one bucket per lane
     __syncwarp();
     // Bucket of every candidate and its rank inside the bucket.
-#pragma unroll 2
+#pragma unroll 1
     for (int t = lane; t < s.len; t += 32) {
       const float4 c = seg[t];
       const float d2 = sq_dist(c.x, c.y, c.z, cx, cy, cz);
@@ -826,7 +865,7 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
     bs[lane] = static_cast<uint16_t>(hi - h);
     if (lane == 31) bs[kBuckets] = static_cast<uint16_t>(hi);
     __syncwarp();
-#pragma unroll 2
+#pragma unroll 1
     for (int t = lane; t < s.len; t += 32) {
       const uint32_t v = w.tmp16[t];
       srt[bs[v >> 10] + (v & 1023u)] = static_cast<uint16_t>(s.seg + t);
@@ -834,13 +873,13 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
     if (lane < ((-s.len) & 7)) srt[s.len + lane] = static_cast<uint16_t>(w.T);  // no candidate
     if (member) {
       const float dx = q.x - cx, dy = q.y - cy, dz = q.z - cz;
-      const float mag = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + sqrtf(far2);
+      const float mag = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) + sqrt_above(far2);
       mapped = true;
       mine.len = cut_accepts_any(a.cut_r2) ? s.len : 0;
       mine.srt = srt;
       mine.bstart = bs;
       mine.inv_w2 = inv_w2;
-      mine.rq = sqrtf(dx * dx + dy * dy + dz * dz);
+      mine.rq = sqrt_above(dx * dx + dy * dy + dz * dz);
       mine.eps = mag * 4e-6f + 1e-30f;
     }
     srt += (s.len + 7) & ~7;
@@ -857,8 +896,9 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
   };
   uint64_t L[KCAP];
   if constexpr (KCAP >= 8) {
-    select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, meta, pop,
-                        popped);
+    const uint32_t none = static_cast<uint32_t>(w.T) * 0x10001u;  // the tile's empty record
+    select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, a, n_items,
+                        none, next);
   } else {
     const int len = mine.len;
 #pragma unroll
@@ -873,13 +913,7 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
     }
     sort_network<KCAP, 0, KCAP>(L);
     uint32_t thr = kth_limit(L[KCAP - 1], cut_lim);
-    auto kth_stop = [&] {
-      const uint64_t last = L[KCAP - 1];
-      return last == kEmpty
-                 ? len
-                 : stop_position(__uint_as_float(static_cast<uint32_t>(last >> 32)), mine);
-    };
-    int stop = len > 0 ? kth_stop() : 0;
+    int stop = len > 0 ? stop_position(__uint_as_float(thr), mine) : 0;
     // Candidate t of the lane's scan: accepted when it beats the K-th.
     auto test = [&](int t, uint64_t& x) {
       float4 c;
@@ -910,29 +944,15 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
       if (any1) list_insert<KCAP>(L, x1);
       if (acc0 || acc1) {
         thr = kth_limit(L[KCAP - 1], cut_lim);
-        stop = min(stop, kth_stop());
+        stop = min(stop, stop_position(__uint_as_float(thr), mine));
       }
     }
-    if (pop) popped = pop_item(meta);
+    next.pop(meta);
+    next.load(a, n_items);
   }
+  next.load_groups(a, n_items, n_groups);
   if (lane < qn && mapped) write_row<IdxT, KCAP, EXACT>(a, L, __float_as_int(q.w), k);
   __syncwarp();
-}
-
-// After a bounded wait gave up: waits once more (bounded) for every buffer
-// that still has bulk copies in flight, so the warp does not leave while the
-// copies write into its shared memory; if they still have not landed, says
-// so with kStatusCopyInFlight.  The warp then stops; the other warps of its
-// CTA (which keep the shared memory allocated) finish their own items.
-__device__ __noinline__ void drain_after_timeout(Meta* meta, const WarpSmem& w, uint32_t phase,
-                                                 uint32_t pending, int depth) {
-  const int lane = threadIdx.x & 31;
-  if (lane == 0) raise_status(&meta->status, kStatusTimeout);
-  bool landed = true;
-  for (int b = 0; b < depth; ++b)
-    if (((pending >> b) & 1u) && !mbar_wait_bounded(w.bar(b), (phase >> b) & 1u, kWaitLimit))
-      landed = false;
-  if (!__all_sync(kFull, landed) && lane == 0) raise_status(&meta->status, kStatusCopyInFlight);
 }
 
 // The persistent query kernel.  Each warp pulls items from the queue; with
@@ -956,60 +976,62 @@ __global__ void __maxnreg__(query_max_regs<KCAP>())
     mbar_init_fence();
   }
   __syncwarp();
-  // bit b: the parity to wait for on buffer b's barrier / copies armed there
-  uint32_t phase = 0u, pending = 0u;
+  uint32_t phase = 0u;  // bit b: the parity to wait for on buffer b's barrier
   const int n_items = meta->n_items;
   const int n_groups = *a.group_count_ptr;
 
+  auto stage = [&](const NextItem& x, int b) {
+    const int staged = x.item < n_items ? stage_item(a, x, n_groups, T, w, b) : -1;
+    copy_async_commit();
+    return staged;
+  };
   int buf = 0;
-  int item = item_of(pop_item(meta));
-  int4 it = load_item(a, item, n_items);
-  int staged = item < n_items ? stage_item(a, it, n_groups, T, w, buf) : -1;
-  if (staged == 1) pending |= 1u << buf;
-  while (item < n_items) {
-    int popped = 0, next = n_items, next_staged = -1;
-    int4 next_it = make_int4(0, 0, 0, 0);
+  NextItem cur{true, 0, 0, make_int4(0, 0, 0, 0), 0, 0, 0};
+  cur.pop(meta);
+  cur.load(a, n_items);
+  cur.load_groups(a, n_items, n_groups);
+  int staged = stage(cur, buf);
+  while (cur.item < n_items) {
+    NextItem next{true, 0, n_items, make_int4(0, 0, 0, 0), 0, 0, 0};
+    int next_staged = -1;
     if (depth > 1) {  // the next item's copies fly while this one is scanned
-      next = item_of(pop_item(meta));
-      next_it = load_item(a, next, n_items);
-      if (next < n_items) next_staged = stage_item(a, next_it, n_groups, T, w, buf ^ 1);
-      if (next_staged == 1) pending |= 1u << (buf ^ 1);
+      next.pop(meta);
+      next.load(a, n_items);
+      next.load_groups(a, n_items, n_groups);
+      next_staged = stage(next, buf ^ 1);
+      next.wanted = false;
     }
+    const int4 it = cur.it;
     if (staged == 1) {
       float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
       if (lane < it.y) q = a.qrec[it.x + lane];  // in flight during the wait
-      if (!mbar_wait_bounded(w.bar(buf), (phase >> buf) & 1u, kWaitLimit)) {
-        drain_after_timeout(meta, w, phase, pending, depth);
-        return;
-      }
-      phase ^= 1u << buf;
-      pending &= ~(1u << buf);
-      packed_item<KCAP, EXACT, IdxT>(a, it, q, w, buf, depth == 1, popped);
+      if (depth > 1)
+        copy_async_wait<1>();
+      else
+        copy_async_wait<0>();
+      __syncwarp();
+      packed_item<KCAP, EXACT, IdxT>(a, it, q, w, buf, n_items, n_groups, next);
     } else {
       if (staged == 0) {
         const int nxt = chunked_item<KCAP, EXACT, IdxT>(a, T, min_cands_per_lane, it.x, it.y, it.z,
                                                         a.k, w.tile(buf), w.hist, w.bar(buf),
                                                         (phase >> buf) & 1u);
-        if (nxt < 0) {  // its own copies were waited for; the other buffer's may fly
-          drain_after_timeout(meta, w, phase, pending, depth);
-          return;
-        }
+        if (nxt < 0) break;  // a bounded wait gave up: its own copies were waited for
         phase = (phase & ~(1u << buf)) | (static_cast<uint32_t>(nxt) << buf);
       }
-      if (depth == 1) popped = pop_item(meta);
+      next.pop(meta);
+      next.load(a, n_items);
+      next.load_groups(a, n_items, n_groups);
     }
-    if (depth > 1) {
+    if (depth > 1)
       buf ^= 1;
-    } else {
-      next = item_of(popped);
-      next_it = load_item(a, next, n_items);
-      if (next < n_items) next_staged = stage_item(a, next_it, n_groups, T, w, buf);
-      if (next_staged == 1) pending |= 1u << buf;
-    }
-    item = next;
-    it = next_it;
+    else
+      next_staged = stage(next, buf);
+    cur = next;
+    cur.wanted = true;
     staged = next_staged;
   }
+  copy_async_wait<0>();  // none in flight when the warp leaves
   __syncwarp();
 }
 
