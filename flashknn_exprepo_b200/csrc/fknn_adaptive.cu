@@ -690,7 +690,6 @@ struct ABufs {
   int32_t* group_row;
   int4* items;
   int32_t* cands;
-  uint32_t* seg_counts;
 };
 
 ABufs alayout(void* ws, int64_t n, size_t* bytes) {
@@ -724,7 +723,6 @@ ABufs alayout(void* ws, int64_t n, size_t* bytes) {
   b.group_row = a.take<int32_t>(n);
   b.items = a.take<int4>(items_capacity(n, n));
   b.cands = a.take<int32_t>(n);
-  b.seg_counts = a.take<uint32_t>(pack_segments(n));
   if (bytes) *bytes = a.used + 256;
   return b;
 }
@@ -798,8 +796,8 @@ int run_adaptive(const AdaptiveArgs& f, void* ws, size_t ws_bytes, const QuerySh
     launch_chained(ka_levels_out, blocks_for(n, 256), 256, 0, s, n, b.rec, b.sel, f.level_out);
     ++nl;
   }
-  nl += launch_items(b.runs, b.group_start, b.group_row, &b.meta->n_groups, n, shape.tile_records,
-                     b.cands, b.seg_counts, &b.meta->n_items, b.items, s, &b.meta->status, n,
+  nl += launch_items(b.runs, b.group_start, b.group_start + 1, b.group_row, &b.meta->n_groups, n,
+                     shape.tile_records, b.cands, &b.meta->n_items, b.items, s, &b.meta->status, n,
                      false);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -813,6 +811,7 @@ int run_adaptive(const AdaptiveArgs& f, void* ws, size_t ws_bytes, const QuerySh
   q.n_qrec = static_cast<int>(n);
   q.runs = b.runs;
   q.group_start = b.group_start;
+  q.group_end = b.group_start + 1;
   q.group_row = b.group_row;
   q.group_count_ptr = &b.meta->n_groups;
   q.items = b.items;

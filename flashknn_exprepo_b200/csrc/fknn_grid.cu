@@ -5,18 +5,20 @@
 // is a fixed sequence of launches with every data-dependent size kept on the
 // device, so it is CUDA-graph capturable:
 //
-//   k_init          zero the Meta block, empty the per-cloud boxes
+//   k_init          zero the Meta block and the cell tables, empty the
+//                   per-cloud boxes
 //   k_bbox          parent cell (grid >> num_down) and cloud of each point,
 //                   range checks, per-cloud bounding boxes (block-aggregated
 //                   atomics)
-//   k_meta          bits per axis of the translated parent coordinates
+//   (k_meta)        bits per axis of the translated parent coordinates; up to
+//                   1,024 clouds the next kernel's CTAs derive them
 //   support cells   counting sort by cell through an open-addressing table
 //                   keyed by cloud << 3*bpa | morton(parent - cloud min):
 //     k_cell_insert   per point its cell's slot and its rank in the cell
 //                     (warp-aggregated count atomics), cell ids in order of
 //                     creation
-//     k_cell_tiles / k_scan_tiles / k_cell_starts
-//                     cell starts in id order, written into the table
+//     k_cell_starts   cell starts (every CTA's cells together, in id order),
+//                     written into the table
 //     k_scatter       float4 records (x, y, z, point id) at start + rank
 //   query groups    general queries: query cells by the same counting sort
 //                   through a second table; selected queries: support cells
@@ -117,12 +119,19 @@ __device__ __forceinline__ int cloud_of(const PointSrc& p, int64_t i, int* statu
 
 // ------------------------------------------------------------------ init
 
-__global__ void k_init(Meta* meta, int* bbox, int64_t n_clouds) {
+// Zeroes the Meta block and the cell tables, empties the per-cloud boxes.
+__global__ void __launch_bounds__(256)
+    k_init(Meta* meta, int* bbox, int64_t n_clouds, uint4* __restrict__ table, size_t slots,
+           uint4* __restrict__ table2, size_t slots2) {
   chain_wait();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  if (t < static_cast<int64_t>(sizeof(Meta) / sizeof(int))) reinterpret_cast<int*>(meta)[t] = 0;
-  for (int64_t i = t; i < n_clouds * 6; i += stride) bbox[i] = (i % 6) < 3 ? INT_MAX : INT_MIN;
+  const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+  if (t < sizeof(Meta) / sizeof(int)) reinterpret_cast<int*>(meta)[t] = 0;
+  for (size_t i = t; i < static_cast<size_t>(n_clouds) * 6; i += stride)
+    bbox[i] = (i % 6) < 3 ? INT_MAX : INT_MIN;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (size_t i = t; i < slots; i += stride) table[i] = zero;
+  for (size_t i = t; i < slots2; i += stride) table2[i] = zero;
 }
 
 // ------------------------------------------------------------------ bbox
@@ -224,10 +233,11 @@ __global__ void __launch_bounds__(256) k_bbox(PointSrc p, int4* __restrict__ pc,
   }
 }
 
-// One CTA: bits per axis of the largest per-cloud extent, batch bits.
-__global__ void __launch_bounds__(1024) k_meta(const int* __restrict__ bbox, int64_t n_clouds,
-                                               Meta* meta) {
-  chain_wait();
+// Bits per axis of the largest per-cloud extent, batch bits: written to the
+// Meta block by the one CTA that is asked to, returned (bits per axis) to every
+// thread of each.
+__device__ __forceinline__ int extent_bits(const int* __restrict__ bbox, int64_t n_clouds,
+                                           Meta* meta, bool write) {
   __shared__ int s_ext[32], s_b[32];
   int ext = 0, maxb = 0;
   for (int64_t c = threadIdx.x; c < n_clouds; c += blockDim.x) {
@@ -244,18 +254,26 @@ __global__ void __launch_bounds__(1024) k_meta(const int* __restrict__ bbox, int
     s_b[threadIdx.x >> 5] = maxb;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
-      ext = max(ext, s_ext[w]);
-      maxb = max(maxb, s_b[w]);
-    }
-    const int bpa = ext > 0 ? 32 - __clz(ext) : 0;
+  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
+    ext = max(ext, s_ext[w]);
+    maxb = max(maxb, s_b[w]);
+  }
+  const int bpa = ext > 0 ? 32 - __clz(ext) : 0;
+  if (write && threadIdx.x == 0) {
     const int bb = maxb > 0 ? 32 - __clz(maxb) : 0;
     meta->bpa = bpa;
     meta->batch_bits = bb;
     meta->max_extent = ext;
     meta->key_bits = 3 * bpa + bb;
   }
+  return bpa;
+}
+
+// The same as a kernel of one CTA, for many clouds.
+__global__ void __launch_bounds__(1024) k_meta(const int* __restrict__ bbox, int64_t n_clouds,
+                                               Meta* meta) {
+  chain_wait();
+  extent_bits(bbox, n_clouds, meta, true);
 }
 
 __device__ __forceinline__ uint64_t cell_key_of(int4 c, const int* bbox, int bpa) {
@@ -281,9 +299,9 @@ __device__ __forceinline__ int axis_offset(int position) {
 // The table also builds the cells, as a counting sort by cell instead of a
 // sort by key.  k_cell_insert counts the points of every cell in its slot
 // and gives each point its rank inside the cell; new cells take ids in
-// creation order (one global atomic per CTA); k_cell_tiles / k_scan_tiles /
-// k_cell_starts lay the cells out in id order; k_scatter writes each point's
-// record at start + rank.  Cell and in-cell order are therefore not
+// creation order (one global atomic per CTA); k_cell_starts lays the cells
+// out; k_scatter writes each point's record at start + rank.  Cell and
+// in-cell order are therefore not
 // deterministic, but nothing downstream depends on them: every query's
 // candidates are the same 27 cells and its top-K is exact under the
 // (distance, index) order.
@@ -307,18 +325,21 @@ __device__ __forceinline__ uint32_t hash_slot(uint64_t key, uint32_t mask) {
 // the same cell key elect one leader, which probes once and adds the group's
 // size to the cell count; slot_of[i] / rank_of[i] = the point's slot and its
 // rank in the cell.  cell_slot[id] = slot of cell id; *cell_count = cells.
+// With `boxes` (the number of clouds) every CTA derives the key layout from
+// the boxes itself and CTA 0 records it in the Meta block; else it is there.
 __global__ void __launch_bounds__(256)
     k_cell_insert(const int4* __restrict__ pc, int64_t n, const int* __restrict__ bbox,
                   Meta* meta, HashSlot* __restrict__ table, uint32_t mask,
                   uint32_t* __restrict__ slot_of, uint32_t* __restrict__ rank_of,
-                  uint32_t* __restrict__ cell_slot, int* cell_count, int ppt) {
+                  uint32_t* __restrict__ cell_slot, int* cell_count, int ppt,
+                  int64_t boxes) {
   chain_wait();
   __shared__ uint32_t s_new;
   __shared__ uint32_t s_base;
   __shared__ uint32_t s_list[2048];
   if (threadIdx.x == 0) s_new = 0u;
+  const int bpa = boxes ? extent_bits(bbox, boxes, meta, blockIdx.x == 0) : meta->bpa;
   __syncthreads();
-  const int bpa = meta->bpa;
   const int lane = threadIdx.x & 31;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * 256 * ppt;
 #pragma unroll 2
@@ -367,36 +388,25 @@ __global__ void __launch_bounds__(256)
   for (uint32_t j = threadIdx.x; j < s_new; j += blockDim.x) cell_slot[s_base + j] = s_list[j];
 }
 
-// Points per 256 x ppt cell ids (ppt per thread): tile_counts[tile].
-__global__ void __launch_bounds__(256)
-    k_cell_tiles(const int* cell_count_ptr, const uint32_t* __restrict__ cell_slot,
-                 const HashSlot* __restrict__ table, uint32_t* __restrict__ tile_counts, int ppt) {
-  chain_wait();
-  __shared__ uint32_t warp_sums[32];
-  __shared__ uint32_t s_total;
-  const int cells = *cell_count_ptr;
-  const int64_t base = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * ppt;
-  uint32_t c = 0;
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-    if (r < ppt && base + r < cells)
-      c += static_cast<uint32_t>(table[cell_slot[base + r]].run.y);
-  block_inclusive_scan(c, warp_sums, &s_total);
-  if (threadIdx.x == 0) tile_counts[blockIdx.x] = s_total;
-}
-
-// Cell starts in id order from the scanned tile counts: the slot's run,
-// cell_key[id], cell_start[id] (cell_start[cells] = n) and, when asked,
-// slot_cell[slot] = id and zero_per_cell[id] = 0.
+// Lays the cells out, 256 x ppt cell ids per CTA (ppt per thread): the CTA
+// takes a stretch of the records with one atomic on *placed (0 before) and its
+// cells follow one another inside it, in id order: the slot's run,
+// cell_key[id], [cell_start[id], cell_end[id]) and, when asked,
+// slot_cell[slot] = id and zero_per_cell[id] = 0.  The order of the CTAs'
+// stretches does not matter, so no scan over them comes first (two launches
+// and a second pass over the table's counts).
 __global__ void __launch_bounds__(256)
     k_cell_starts(const int* cell_count_ptr, const uint32_t* __restrict__ cell_slot,
-                  HashSlot* __restrict__ table, const uint32_t* __restrict__ tile_offsets,
-                  int64_t n, uint64_t* __restrict__ cell_key, int32_t* __restrict__ cell_start,
+                  HashSlot* __restrict__ table, int* placed, uint64_t* __restrict__ cell_key,
+                  int32_t* __restrict__ cell_start, int32_t* __restrict__ cell_end,
                   uint32_t* __restrict__ slot_cell, uint32_t* __restrict__ zero_per_cell, int ppt) {
   chain_wait();
   __shared__ uint32_t warp_sums[32];
+  __shared__ uint32_t s_total;
+  __shared__ int s_base;
   const int cells = *cell_count_ptr;
   const int64_t base = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * ppt;
+  if (static_cast<int64_t>(blockIdx.x) * 256 * ppt >= cells) return;  // the whole CTA
   uint32_t cnt[8], slot[8], sum = 0;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
@@ -408,8 +418,10 @@ __global__ void __launch_bounds__(256)
     }
     sum += cnt[r];
   }
-  const uint32_t incl = block_inclusive_scan(sum, warp_sums, nullptr);
-  uint32_t start = tile_offsets[blockIdx.x] + incl - sum;
+  const uint32_t incl = block_inclusive_scan(sum, warp_sums, &s_total);
+  if (threadIdx.x == 0) s_base = atomicAdd(placed, static_cast<int>(s_total));
+  __syncthreads();
+  uint32_t start = static_cast<uint32_t>(s_base) + incl - sum;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     const int64_t c = base + r;
@@ -421,7 +433,7 @@ __global__ void __launch_bounds__(256)
     if (slot_cell) slot_cell[slot[r]] = static_cast<uint32_t>(c);
     if (zero_per_cell) zero_per_cell[c] = 0u;
     start += cnt[r];
-    if (c == cells - 1) cell_start[cells] = static_cast<int32_t>(n);
+    cell_end[c] = static_cast<int32_t>(start);
   }
 }
 
@@ -659,13 +671,14 @@ struct Bufs {
   int32_t* cell_of;
   uint64_t* cell_key;
   int32_t* cell_start;
+  int32_t* cell_end;
   int2* runs;
   uint64_t* group_key;
   int32_t* group_start;
+  int32_t* group_end;
   int32_t* group_row;
   int4* items;
   int32_t* cands;
-  uint32_t* seg_counts;
   HashSlot* hslots;
   int64_t hash_cap;
   uint32_t* slot_cell;  // cell id of each occupied slot (selected queries)
@@ -691,7 +704,8 @@ Bufs layout(void* ws, int64_t n, int64_t m, int64_t n_clouds, int kind, size_t* 
   b.tile_counts2 = a.take<uint32_t>(static_cast<size_t>(ceil_div(nm > 0 ? nm : 1, 2048)));
   b.srec = a.take<float4>(n);
   b.cell_key = a.take<uint64_t>(n);
-  b.cell_start = a.take<int32_t>(n + 1);
+  b.cell_start = a.take<int32_t>(n);
+  b.cell_end = a.take<int32_t>(n);
   b.hash_cap = 16;
   while (b.hash_cap < 2 * n) b.hash_cap <<= 1;
   b.hslots = a.take<HashSlot>(b.hash_cap);
@@ -714,13 +728,13 @@ Bufs layout(void* ws, int64_t n, int64_t m, int64_t n_clouds, int kind, size_t* 
   if (kind != FKNN_QUERY_SELF) {
     b.qrec = a.take<float4>(m);
     b.group_start = a.take<int32_t>(m + 1);
+    if (kind == FKNN_QUERY_GENERAL) b.group_end = a.take<int32_t>(m);
     b.group_row = kind == FKNN_QUERY_SELECTED ? a.take<int32_t>(m) : nullptr;
   }
   const int64_t q = kind == FKNN_QUERY_SELF ? n : m;
   const int64_t max_groups = kind == FKNN_QUERY_SELF ? n : m;
   b.items = a.take<int4>(items_capacity(max_groups, q));
   b.cands = a.take<int32_t>(max_groups);
-  b.seg_counts = a.take<uint32_t>(pack_segments(max_groups));
   if (bytes) *bytes = a.used + 256;
   return b;
 }
@@ -777,7 +791,12 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
   cudaError_t e;
   const uint32_t hmask = static_cast<uint32_t>(b.hash_cap - 1);
 
-  launch_chained(k_init, 64, 256, 0, s, b.meta, b.bbox, n_clouds);
+  const bool qtable = kind == FKNN_QUERY_GENERAL && m > 0;
+  const size_t slots = n > 0 ? static_cast<size_t>(b.hash_cap) : 0;
+  const size_t qslots = qtable ? static_cast<size_t>(b.qhash_cap) : 0;
+  launch_chained(k_init, capped_blocks(static_cast<int64_t>(slots + qslots) / 4 + 1), 256, 0, s,
+                 b.meta, b.bbox, n_clouds, reinterpret_cast<uint4*>(b.hslots), slots,
+                 reinterpret_cast<uint4*>(b.qslots), qslots);
   ++nl;
 
   const float inv_voxel = 1.0f / f.voxel;  // host FP32 division, correctly rounded
@@ -797,28 +816,27 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
                    ppt_q);
     ++nl;
   }
-  launch_chained(k_meta, 1, 1024, 0, s, b.bbox, n_clouds, b.meta);
-  ++nl;
+  // Up to 1,024 clouds every CTA of the first insertion reads the boxes
+  // itself (four or fewer per thread); more are reduced once by a kernel.
+  int64_t boxes = n_clouds <= 1024 ? n_clouds : 0;
+  if (!boxes) {
+    launch_chained(k_meta, 1, 1024, 0, s, b.bbox, n_clouds, b.meta);
+    ++nl;
+  }
 
   // --- support cells
   if (n > 0) {
     // Counting sort by cell through the hash table.
-    e = cudaMemsetAsync(b.hslots, 0, sizeof(HashSlot) * static_cast<size_t>(b.hash_cap), s);
-    if (e != cudaSuccess) {
-      note_cuda_error(e);
-      return FKNN_ERR_CUDA;
-    }
     const int tiles = blocks_for(n, 256 * ppt_s);
     launch_chained(k_cell_insert, tiles, 256, 0, s, b.pc_s, n, b.bbox, b.meta, b.hslots, hmask,
-                   b.slot_of, b.rank_of, b.cell_slot, &b.meta->n_cells, ppt_s);
-    launch_chained(k_cell_tiles, tiles, 256, 0, s,
-        &b.meta->n_cells, b.cell_slot, b.hslots, b.tile_counts, ppt_s);
-    launch_chained(k_scan_tiles, 1, 1024, 0, s, b.tile_counts, tiles, &b.meta->n_points_scanned);
+                   b.slot_of, b.rank_of, b.cell_slot, &b.meta->n_cells, ppt_s, boxes);
+    boxes = 0;
     launch_chained(k_cell_starts, tiles, 256, 0, s, &b.meta->n_cells, b.cell_slot, b.hslots,
-                   b.tile_counts, n, b.cell_key, b.cell_start, b.slot_cell, b.qcount, ppt_s);
+                   &b.meta->n_points_scanned, b.cell_key, b.cell_start, b.cell_end, b.slot_cell,
+                   b.qcount, ppt_s);
     launch_chained(k_scatter, blocks_for(n, 256), 256, 0, s, f.xyz, f.sindex, f.n_src, n, b.slot_of,
         b.rank_of, b.hslots, b.slot_cell, b.srec, b.pos_of, b.cell_of, &b.meta->status);
-    nl += 5;
+    nl += 3;
   }
 
   const float4* qrec = b.srec;
@@ -827,6 +845,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
   int pad_mode = f.pad_minus_one ? kPadMinusOne : kPadSelf;
   const void* pad = nullptr;
   const int32_t* group_start = b.cell_start;
+  const int32_t* group_end = b.cell_end;
   const int32_t* group_row = nullptr;
   const int* group_count_ptr = &b.meta->n_cells;
 
@@ -836,9 +855,9 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
                      &b.meta->status);
       ++nl;
-      nl += launch_items(b.runs, b.cell_start, nullptr, &b.meta->n_cells, n, shape.tile_records,
-                         b.cands, b.seg_counts, &b.meta->n_items, b.items, s, &b.meta->status, n,
-                         true);
+      nl += launch_items(b.runs, b.cell_start, b.cell_end, nullptr, &b.meta->n_cells, n,
+                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
+                         &b.meta->status, n, true);
     }
   } else if (kind == FKNN_QUERY_SELECTED) {
     pad_mode = kPadArray64;
@@ -846,6 +865,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     qrec = b.qrec;
     n_qrec = static_cast<int>(m);
     group_start = b.group_start;
+    group_end = b.group_start + 1;
     group_row = b.group_row;
     group_count_ptr = &b.meta->n_groups;
     if (n > 0) {
@@ -870,8 +890,8 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
       launch_chained(k_sel_scatter, blocks_for(m, 256), 256, 0, s, m, n, f.query_indices, b.pos_of,
           b.srec, b.slot_of, b.rank_of, b.qstart, b.qrec, &b.meta->status);
       nl += 6;
-      nl += launch_items(b.runs, b.group_start, b.group_row, &b.meta->n_groups, m,
-                         shape.tile_records, b.cands, b.seg_counts, &b.meta->n_items, b.items, s,
+      nl += launch_items(b.runs, b.group_start, group_end, b.group_row, &b.meta->n_groups, m,
+                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
                          &b.meta->status, m, false);
     }
   } else {  // general queries
@@ -880,35 +900,29 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     n_qrec = static_cast<int>(m);
     runs = b.runs;
     group_start = b.group_start;
+    group_end = b.group_end;
     group_count_ptr = &b.meta->n_groups;
     if (m > 0) {
       // query groups = query cells, by the same counting sort through a
       // second table (slot_of / rank_of / cell_slot are free again once the
       // support records are written)
-      e = cudaMemsetAsync(b.qslots, 0, sizeof(HashSlot) * static_cast<size_t>(b.qhash_cap), s);
-      if (e != cudaSuccess) {
-        note_cuda_error(e);
-        return FKNN_ERR_CUDA;
-      }
       const uint32_t qmask = static_cast<uint32_t>(b.qhash_cap - 1);
       const int tiles = blocks_for(m, 256 * ppt_q);
       launch_chained(k_cell_insert, tiles, 256, 0, s, b.pc_q, m, b.bbox, b.meta, b.qslots, qmask,
-          b.slot_of, b.rank_of, b.cell_slot, &b.meta->n_groups, ppt_q);
-      launch_chained(k_cell_tiles, tiles, 256, 0, s,
-          &b.meta->n_groups, b.cell_slot, b.qslots, b.tile_counts, ppt_q);
-      launch_chained(k_scan_tiles, 1, 1024, 0, s, b.tile_counts, tiles, &b.meta->n_points_scanned);
+          b.slot_of, b.rank_of, b.cell_slot, &b.meta->n_groups, ppt_q, boxes);
       launch_chained(k_cell_starts, tiles, 256, 0, s, &b.meta->n_groups, b.cell_slot, b.qslots,
-                     b.tile_counts, m, b.group_key, b.group_start, nullptr, nullptr, ppt_q);
+                     &b.meta->reserved[0], b.group_key, b.group_start, b.group_end, nullptr,
+                     nullptr, ppt_q);
       launch_chained(k_scatter, blocks_for(m, 256), 256, 0, s, f.qxyz, nullptr, m, m, b.slot_of,
           b.rank_of, b.qslots, nullptr, b.qrec, nullptr, nullptr, &b.meta->status);
-      nl += 5;
+      nl += 3;
       launch_chained(k_runs, capped_blocks(m * 32), 256, 0, s, b.group_key, &b.meta->n_groups,
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
                      &b.meta->status);
       ++nl;
-      nl += launch_items(b.runs, b.group_start, nullptr, &b.meta->n_groups, m, shape.tile_records,
-                         b.cands, b.seg_counts, &b.meta->n_items, b.items, s, &b.meta->status, m,
-                         true);
+      nl += launch_items(b.runs, b.group_start, b.group_end, nullptr, &b.meta->n_groups, m,
+                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
+                         &b.meta->status, m, true);
     }
   }
 
@@ -925,6 +939,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     q.n_qrec = n_qrec;
     q.runs = runs;
     q.group_start = group_start;
+    q.group_end = group_end;
     q.group_row = group_row;
     q.group_count_ptr = group_count_ptr;
     q.items = b.items;

@@ -22,8 +22,8 @@ struct Meta {
   int qkey_bits;    // significant bits of the selected-query cell keys
   int batch_bits;   // bits of the largest batch id
   int max_extent;   // largest per-cloud parent-coordinate extent
-  int n_points_scanned;  // total of a scan over per-cell point counts (= n)
-  int reserved[3];  // per-path scratch words (the adaptive octree's)
+  int n_points_scanned;  // support records laid out so far (= n at the end)
+  int reserved[3];  // per-path scratch words (the adaptive octree's, [0]: query records laid out)
   // sum over the query groups of their 27-cell candidate totals (self and
   // general queries; read back for FlashKNN.query's traverse_info)
   unsigned long long cand_total;
@@ -58,7 +58,8 @@ struct QueryLaunch {
   const float4* qrec;  // query records (x, y, z, output-row bits)
   int n_qrec;
   const int2* runs;    // [rows][27] (start, count) into srec
-  const int32_t* group_start;  // [groups + 1] query ranges in qrec
+  const int32_t* group_start;  // query range of each group in qrec
+  const int32_t* group_end;
   const int32_t* group_row;    // runs row of each group, or null (row = group)
   const int* group_count_ptr;  // device: number of groups
   const int4* items;   // work items (see above)
@@ -78,11 +79,12 @@ struct QueryLaunch {
 int launch_query(const QueryLaunch& q, const QueryShape& shape, cudaStream_t s);
 
 // Item construction (fknn_items.cu): per-group candidate counts, segmented
-// greedy packing; *n_items_ptr receives the item count.  Returns launches.
-int launch_items(const int2* runs, const int32_t* group_start, const int32_t* group_row,
-                 const int* group_count_ptr, int64_t max_groups, int tile, int32_t* cands,
-                 uint32_t* seg_counts, int* n_items_ptr, int4* items, cudaStream_t s,
-                 int* status, int64_t n_queries, bool cands_ready);
+// greedy packing; *n_items_ptr (0 before) receives the item count.  Group g's
+// queries are the records [group_start[g], group_end[g]).  Returns launches.
+int launch_items(const int2* runs, const int32_t* group_start, const int32_t* group_end,
+                 const int32_t* group_row, const int* group_count_ptr, int64_t max_groups, int tile,
+                 int32_t* cands, int* n_items_ptr, int4* items, cudaStream_t s, int* status,
+                 int64_t n_queries, bool cands_ready);
 size_t items_capacity(int64_t max_groups, int64_t n_queries);
 // Bounded-wait self-test (fknn_selftest.cu): arms a barrier that never
 // completes and waits at most `limit` polls; sets kStatusTimeout.
@@ -100,7 +102,7 @@ __host__ __device__ inline int pack_segment_len(int n_groups) {
   const int len = n_groups / kPackWarps;
   return len < kPackSegmentMin ? kPackSegmentMin : len;
 }
-// Segment counts to allocate for up to max_groups groups (every length).
+// Segments of up to max_groups groups (every length).
 inline int64_t pack_segments(int64_t max_groups) {
   return (max_groups + kPackSegmentMin - 1) / kPackSegmentMin;
 }

@@ -264,7 +264,7 @@ struct NextItem {
     const int g = it.z + lane;
     if (it.z >= 0 && it.z < n_groups && lane < (it.w & 0xffff) && g < n_groups) {
       gs = a.group_start[g];
-      ge = a.group_start[g + 1];
+      ge = a.group_end[g];
       row = a.group_row ? a.group_row[g] : g;
     }
   }
@@ -472,11 +472,12 @@ __device__ __forceinline__ int2 load_run(const QueryLaunch& a, int row, int lane
 // qlist: 32 ints of scratch; hist: 8 counters.  Kept out of line so its
 // registers do not add to the packed path's.
 __device__ __noinline__ int ordered_query_row(const float4* __restrict__ qrec,
-                                              const int32_t* __restrict__ group_start, int g0,
+                                              const int32_t* __restrict__ group_start,
+                                              const int32_t* __restrict__ group_end, int g0,
                                               int q0, int qn, int qi, bool active, int* qlist,
                                               uint32_t* hist) {
   const int lane = threadIdx.x & 31;
-  const int gq0 = group_start[g0], gq1 = group_start[g0 + 1];
+  const int gq0 = group_start[g0], gq1 = group_end[g0];
   const int nqg = gq1 - gq0;
   if (!(nqg > qn && nqg <= kMaxOrderedGroup && q0 >= gq0 && q0 + qn <= gq1))
     return q0 + qi;
@@ -566,7 +567,7 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
   // them instead in octant-major order
   // (ordered_query_row), so an item's queries are close together and the
   // phase-B sphere below stays small.
-  const int qrow = ordered_query_row(a.qrec, a.group_start, g0, q0, qn, qi, active,
+  const int qrow = ordered_query_row(a.qrec, a.group_start, a.group_end, g0, q0, qn, qi, active,
                                      reinterpret_cast<int*>(tile), hist);
   float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
   if (active) q = a.qrec[qrow];

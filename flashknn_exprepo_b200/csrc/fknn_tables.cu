@@ -120,7 +120,6 @@ struct TabBufs {
   int2* runs;
   int4* items;
   int32_t* cands;
-  uint32_t* seg_counts;
 };
 
 TabBufs tab_layout(void* ws, int64_t n, int64_t m, int64_t p, size_t* bytes) {
@@ -132,7 +131,6 @@ TabBufs tab_layout(void* ws, int64_t n, int64_t m, int64_t p, size_t* bytes) {
   b.runs = a.take<int2>(static_cast<size_t>(p) * 27);
   b.items = a.take<int4>(items_capacity(p, m));
   b.cands = a.take<int32_t>(p);
-  b.seg_counts = a.take<uint32_t>(pack_segments(p));
   if (bytes) *bytes = a.used + 256;
   return b;
 }
@@ -174,10 +172,11 @@ int run_tables(const TablesArgs& t, void* ws, size_t ws_bytes, const QueryShape&
                    b.meta, b.qrec);
     ++nl;
   }
+  const int32_t* steps = selected ? t.steps_query : t.steps;
   if (t.p > 0)
-    nl += launch_items(b.runs, selected ? t.steps_query : t.steps, nullptr, &b.meta->n_groups, t.p,
-                       shape.tile_records, b.cands, b.seg_counts, &b.meta->n_items, b.items, s,
-                       &b.meta->status, selected ? m : t.n, false);
+    nl += launch_items(b.runs, steps, steps + 1, nullptr, &b.meta->n_groups, t.p,
+                       shape.tile_records, b.cands, &b.meta->n_items, b.items, s, &b.meta->status,
+                       selected ? m : t.n, false);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     note_cuda_error(e);
@@ -190,7 +189,8 @@ int run_tables(const TablesArgs& t, void* ws, size_t ws_bytes, const QueryShape&
     q.qrec = selected ? b.qrec : b.srec;
     q.n_qrec = static_cast<int>(m);
     q.runs = b.runs;
-    q.group_start = selected ? t.steps_query : t.steps;
+    q.group_start = steps;
+    q.group_end = steps + 1;
     q.group_row = nullptr;
     q.group_count_ptr = &b.meta->n_groups;
     q.items = b.items;

@@ -1,0 +1,52 @@
+"""Cells laid out by one atomic per CTA and items placed by another, where the
+pieces meet: cell counts around a CTA's share, runs of items that must not
+span a gap between two CTAs' records, many clouds (the key layout read by
+every CTA up to 1,024 of them, by one kernel beyond) -- bit-exact against the
+oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _points(rng, cells):
+    """One to three points in each of `cells` voxels of 1 in a slab."""
+    w = int(np.ceil(np.sqrt(cells)))
+    at = np.stack(np.meshgrid(np.arange(w), np.arange(w), indexing="ij"), -1).reshape(-1, 2)[:cells]
+    reps = rng.integers(1, 4, cells)
+    xy = np.repeat(at, reps, 0) + rng.random((reps.sum(), 2))
+    xyz = np.concatenate([xy, rng.random((len(xy), 1))], 1).astype(np.float32)
+    rng.shuffle(xyz)
+    return np.ascontiguousarray(xyz)
+
+
+def _check(xyz, offs, k, new=None, new_offs=None):
+    import flashknn_exprepo_b200 as fk
+    oi, od = O.knn_offsets(xyz, offs, k, 0.25, 2, new, new_offs)
+    to = lambda a: None if a is None else torch.from_numpy(a).to(DEV)
+    gi, gd = fk.ops.knn_offsets(to(xyz), to(offs), k, 0.25, 2, to(new), to(new_offs),
+                                validate=True)
+    assert np.array_equal(gi.cpu().numpy(), oi)
+    assert np.array_equal(gd.cpu().numpy().view(np.uint32), od.view(np.uint32))
+
+
+@pytest.mark.parametrize("cells", [1, 255, 256, 257, 1023, 2049, 40000])
+def test_cell_counts_around_a_share(cells):
+    rng = np.random.default_rng(cells)
+    xyz = _points(rng, cells)
+    new = _points(rng, max(1, cells // 2))
+    _check(xyz, np.array([len(xyz)]), 8)
+    _check(xyz, np.array([len(xyz)]), 3, new, np.array([len(new)]))
+
+
+@pytest.mark.parametrize("clouds", [1023, 1024, 1025, 3000])
+def test_many_clouds(clouds):
+    rng = np.random.default_rng(clouds)
+    counts = rng.integers(1, 20, clouds)
+    xyz = (rng.random((counts.sum(), 3)) * rng.choice([1, 1, 1, 9], counts.sum())[:, None])
+    _check(np.ascontiguousarray(xyz, dtype=np.float32), np.cumsum(counts).astype(np.int64), 4)
