@@ -42,6 +42,22 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Queries of a chunked item of a group with c candidates.  In a large problem
+// (max_qc = 32) max_qc up to kChunkedFull candidates, then fewer in inverse
+// proportion, at least kChunkedFew: an item's time grows with c, and with full
+// items the heaviest ones (13 thousand candidates) ran on for twice the mean
+// after the others had ended.  A LiDAR scan with 40 cm cells (115 thousand
+// queries) takes 325 us at K=16 and 547 us at K=32, with full items 480 and
+// 728 us; from 1,024 candidates on, or down to 4 queries, it is slower (329 to
+// 382 and 549 to 661 us).  A smaller problem is cut to two items per warp
+// already (chunked_query_cap) and keeps that size: cut further, the DeLA
+// levels gained nothing.
+constexpr int kChunkedFull = 2048, kChunkedFew = 8;
+__device__ __forceinline__ int chunked_queries(int max_qc, int c) {
+  if (c <= kChunkedFull || max_qc < 32) return max_qc;
+  return max(static_cast<int>(static_cast<int64_t>(max_qc) * kChunkedFull / c), kChunkedFew);
+}
+
 // One warp per segment of consecutive groups.  Item = (q_start, q_count,
 // g_first, g_count | flags).
 // The segment's group ranges and candidate counts are loaded once (one
@@ -108,11 +124,12 @@ __global__ void __launch_bounds__(256)
         if (ge <= gs) continue;
         if (c > tile) {  // streams its candidates: items of its own
           flush();
-          const int n_it = (ge - gs + max_qc - 1) / max_qc;
+          const int qc = chunked_queries(max_qc, c);
+          const int n_it = (ge - gs + qc - 1) / qc;
           if (write)
             for (int t = lane; t < n_it; t += 32) {
-              const int q = gs + t * max_qc;
-              put(count + t, q, min(max_qc, ge - q), g, 1, kItemChunked);
+              const int q = gs + t * qc;
+              put(count + t, q, min(qc, ge - q), g, 1, kItemChunked);
             }
           count += n_it;
           continue;
