@@ -19,9 +19,8 @@
 //     centre of the group's queries, so every lane meets near candidates
 //     first and stops at the first bucket whose lower distance bound exceeds
 //     its current K-th distance (triangle inequality, with a safety margin
-//     for FP32 rounding).  Lists of 8 and more take the candidates in blocks
-//     sorted and merged as 32-bit keys (select_blocks); shorter ones insert
-//     them one by one when some lane improves (warp vote);
+//     for FP32 rounding).  The candidates are taken in blocks, sorted and
+//     merged into the lane's list as 32-bit keys (select_blocks);
 //   * chunked item: one group with more candidates than a tile; G lanes per
 //     query split its candidates, streamed tile by tile by non-multicast
 //     cp.async.bulk copies on the warp's mbarrier, and the G partial
@@ -107,38 +106,12 @@ __device__ __forceinline__ void list_insert(uint64_t (&L)[KCAP], uint64_t x) {
   L[0] = key_min(x, L[0]);
 }
 
-// The same network over the upper half only: valid when x does not belong
-// in the lower half (x >= L[KCAP/2 - 1]), which leaves that half unchanged.
-template <int KCAP>
-__device__ __forceinline__ void list_insert_upper(uint64_t (&L)[KCAP], uint64_t x) {
-#pragma unroll
-  for (int j = KCAP - 1; j >= KCAP / 2; --j) {
-    const bool cj = key_less(x, L[j]);
-    const bool cm = key_less(x, L[j - 1]);
-    L[j] = cj ? (cm ? L[j - 1] : x) : L[j];
-  }
-}
-
 template <int KCAP>
 __device__ __forceinline__ void cas(uint64_t (&L)[KCAP], int i, int j, bool ascending) {
   const uint64_t a = L[i], b = L[j];
   const bool sw = ascending ? key_less(b, a) : key_less(a, b);
   L[i] = sw ? b : a;
   L[j] = sw ? a : b;
-}
-
-// Inserts x (kEmpty = none).  Late improvements mostly belong in the upper
-// half of the list: when that holds for every lane, only that half is
-// updated.
-template <int KCAP>
-__device__ __forceinline__ void insert_one(uint64_t (&L)[KCAP], uint64_t x) {
-  if constexpr (KCAP >= 8) {
-    if (__all_sync(kFull, !key_less(x, L[KCAP / 2 - 1]))) {
-      list_insert_upper<KCAP>(L, x);
-      return;
-    }
-  }
-  list_insert<KCAP>(L, x);
 }
 
 template <int KCAP>
@@ -308,7 +281,8 @@ __device__ __forceinline__ void merge_block(uint32_t (&L)[KCAP], const uint32_t 
 // instruction).  With staging and sort the whole call over the 16-cloud batch
 // (1.46 million queries, K=16) went from 861 to 574 us, over 700 thousand
 // queries at K=32 from 880 to 484 us, over 300 thousand at K=64 from 1182 to
-// 522 us.  The keys
+// 522 us.  Short lists gain the same way: 300 thousand queries at K=3 125 ->
+// 100 us, 700 thousand at K=1 323 -> 307 us.  The keys
 // drop the low 9 or 10 bits of the distance, so the exact keys of the list
 // are computed at the end and neighbours that the truncation left in the
 // wrong order are exchanged; a lane whose k-th entry shares its truncated
@@ -320,6 +294,7 @@ __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGro
                                               DistBits& dist_bits, const QueryLaunch& a,
                                               int n_items, uint32_t none, NextItem& next) {
   constexpr int B = KCAP <= 16 ? 8 : 16;
+  constexpr int M = KCAP < B ? KCAP : B;  // of a block that the list can take
   const uint16_t* srt = g.srt;
   uint32_t L[KCAP];
   uint32_t dropped = kNone32, last = kNone32;
@@ -343,7 +318,11 @@ __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGro
     }
     sort_network<B, 0, B>(X);
     if (__any_sync(kFull, X[0] < last)) {
-      merge_block<KCAP, B>(L, X, dropped);
+      uint32_t Y[M];
+#pragma unroll
+      for (int j = 0; j < M; ++j) Y[j] = X[j];
+      if (M < B) dropped = min(dropped, X[M % B]);
+      merge_block<KCAP, M>(L, Y, dropped);
       last = L[KCAP - 1];
       if (k < KCAP) {
 #pragma unroll
@@ -896,61 +875,9 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
     return __float_as_uint(sq_dist(c.x, c.y, c.z, q.x, q.y, q.z));
   };
   uint64_t L[KCAP];
-  if constexpr (KCAP >= 8) {
-    const uint32_t none = static_cast<uint32_t>(w.T) * 0x10001u;  // the tile's empty record
-    select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, a, n_items,
-                        none, next);
-  } else {
-    const int len = mine.len;
-#pragma unroll
-    for (int j = 0; j < KCAP; ++j) {
-      uint64_t key = kEmpty;
-      if (j < len) {
-        float4 c;
-        const uint32_t d = dist_bits(mine.srt[j], c);
-        if (d <= cut_lim) key = make_key(__uint_as_float(d), c.w);
-      }
-      L[j] = key;
-    }
-    sort_network<KCAP, 0, KCAP>(L);
-    uint32_t thr = kth_limit(L[KCAP - 1], cut_lim);
-    int stop = len > 0 ? stop_position(__uint_as_float(thr), mine) : 0;
-    // Candidate t of the lane's scan: accepted when it beats the K-th.
-    auto test = [&](int t, uint64_t& x) {
-      float4 c;
-      const uint32_t d = dist_bits(mine.srt[t], c);
-      const bool acc = d <= thr;
-      if (acc) x = make_key(__uint_as_float(d), c.w);
-      return acc;
-    };
-    // Two candidates per iteration, both tested against the same K-th
-    // distance: half the loop and vote overhead, and two independent loads
-    // and distance chains in flight.
-    for (int t = KCAP;; t += 2) {
-      const bool live0 = t < stop, live1 = t + 1 < stop;
-      if (!__any_sync(kFull, live0)) break;
-      uint64_t x0 = kEmpty, x1 = kEmpty;
-      const bool acc0 = live0 && test(t, x0);
-      const bool acc1 = live1 && test(t + 1, x1);
-      // A lane that took only its second candidate inserts it in the first
-      // step, so the second step runs only when some lane took both (the
-      // list keeps the K smallest of what it is given, in any order).
-      if (!acc0) {
-        x0 = x1;
-        x1 = kEmpty;
-      }
-      const bool any0 = __any_sync(kFull, acc0 || acc1);
-      const bool any1 = __any_sync(kFull, acc0 && acc1);
-      if (any0) list_insert<KCAP>(L, x0);
-      if (any1) list_insert<KCAP>(L, x1);
-      if (acc0 || acc1) {
-        thr = kth_limit(L[KCAP - 1], cut_lim);
-        stop = min(stop, stop_position(__uint_as_float(thr), mine));
-      }
-    }
-    next.pop(meta);
-    next.load(a, n_items);
-  }
+  const uint32_t none = static_cast<uint32_t>(w.T) * 0x10001u;  // the tile's empty record
+  select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, a, n_items, none,
+                      next);
   next.load_groups(a, n_items, n_groups);
   if (lane < qn && mapped) write_row<IdxT, KCAP, EXACT>(a, L, __float_as_int(q.w), k);
   __syncwarp();

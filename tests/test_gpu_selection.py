@@ -38,7 +38,7 @@ def _lattice(side, jitter):
 
 
 @pytest.mark.parametrize("jitter", [0.0, 2e-6, 2e-5, 1e-3])
-@pytest.mark.parametrize("k", [5, 8, 9, 16, 17, 24, 32, 33, 64])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 16, 17, 24, 32, 33, 64])
 def test_distance_classes(k, jitter):
     _check(_lattice(17, jitter), k, 0.5)
 
@@ -52,7 +52,7 @@ def test_wide_tile_positions(k):
         _check(xyz, k, voxel, _lib.FknnConfig(2, 512, 8, 0, 2))
 
 
-@pytest.mark.parametrize("k", [5, 8, 16, 24])
+@pytest.mark.parametrize("k", [1, 3, 5, 8, 16, 24])
 def test_candidate_counts_around_a_block(k):
     """Cells far apart, each its own neighbourhood of 1..70 points, some of
     them duplicates."""
