@@ -23,7 +23,14 @@ struct Meta {
   int batch_bits;   // bits of the largest batch id
   int max_extent;   // largest per-cloud parent-coordinate extent
   int n_points_scanned;  // support records laid out so far (= n at the end)
-  int reserved[3];  // per-path scratch words (the adaptive octree's, [0]: query records laid out)
+  // per-path scratch words
+  union {
+    int reserved[3];  // the adaptive octree's
+    struct {
+      int n_queries_placed;  // query records laid out so far (general queries)
+      int last_cloud;        // largest cloud id of any point
+    };
+  };
   // sum over the query groups of their 27-cell candidate totals (self and
   // general queries; read back for FlashKNN.query's traverse_info)
   unsigned long long cand_total;
