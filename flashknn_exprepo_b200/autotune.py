@@ -6,7 +6,7 @@ per warp (``tile_records``; groups with more candidates stream tile by
 tile), how many lanes may share one query when a group is larger than a
 tile (``min_candidates_per_lane``), and the shared-memory staging depth (1:
 a warp stages a work item's candidates and then scans them; 2: two tiles
-per warp, the next item's bulk copies in flight during the scan, at twice
+per warp, the next item's copies in flight during the scan, at twice
 the tile memory, hence fewer resident warps).  The best shape depends on K (register
 list length, hence occupancy) and on point density (candidates per query,
 hence tile fill and the chunked path).  ``tune_offsets`` times a

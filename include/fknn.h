@@ -64,7 +64,7 @@ extern "C" {
  * min_candidates_per_lane >= 1 caps how many lanes share one query;
  * ctas_per_sm 0 = occupancy maximum; staging_depth 1 (stage a work item's
  * candidates, then scan them) or 2 (two tiles per warp: the next item's
- * bulk copies are in flight while the current one is scanned).  Zero
+ * copies are in flight while the current one is scanned).  Zero
  * fields take the defaults.  flashknn_exprepo_b200/autotune.py picks these
  * per K and point density by timing them. */
 typedef struct fknn_config {
