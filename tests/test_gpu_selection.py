@@ -64,3 +64,15 @@ def test_candidate_counts_around_a_block(k):
     xyz = np.ascontiguousarray(np.concatenate([xyz, xyz[dup]]))
     _check(xyz, k, 0.1)
     _check(xyz, k, 0.1, cut_r2=0.01)
+
+
+@pytest.mark.parametrize("radius", [0.25, 99999.0, 100001.0, 4e5])
+def test_ball_padding_on_both_sides_of_its_radius_rule(radius):
+    import flashknn_exprepo_b200 as fk
+    rng = np.random.default_rng(7)
+    xyz = torch.from_numpy((rng.random((300, 3)) * 4 * radius).astype(np.float32)).to(DEV)
+    offs = torch.tensor([300], device=DEV)
+    idx, dist = fk.ball_query(24, radius, 0.0, xyz, offs)
+    want_idx, d2 = fk.ops.ball_query_offsets(xyz, offs, 24, radius, radius / 4, 2, None, None)
+    assert torch.equal(idx, want_idx) and bool((idx < 0).any()) and bool((idx >= 0).any())
+    assert torch.equal(dist, torch.where(idx < 0, torch.full_like(d2, 1e5), torch.sqrt(d2)))
