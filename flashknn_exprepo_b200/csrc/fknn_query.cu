@@ -595,8 +595,10 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
           float4 c = q;
           if (t < cnt) {
             c = tile[t];
+            // NaN keeps the candidate: one query with a NaN coordinate makes the
+            // centroid NaN, and the item's other queries still need them all
             const float dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
-            keep = dx * dx + dy * dy + dz * dz <= rad2;
+            keep = !(dx * dx + dy * dy + dz * dz > rad2);
           }
           // in place: the kept records move towards the front, never past
           // the ones still to be read (the ballot follows every lane's read)
