@@ -601,8 +601,10 @@ __device__ __noinline__ int chunked_item(const QueryLaunch& a, int T, int min_ca
             keep = !(dx * dx + dy * dy + dz * dz > rad2);
           }
           // in place: the kept records move towards the front, never past
-          // the ones still to be read (the ballot follows every lane's read)
+          // the ones still to be read; a vote orders no memory, so the warp
+          // barrier keeps this step's reads before its stores
           const uint32_t b = __ballot_sync(kFull, keep);
+          __syncwarp();
           if (keep) tile[m + __popc(b & lanemask_lt())] = c;
           m += __popc(b);
         }
