@@ -159,37 +159,12 @@ struct Acc {
   float x = 0.f, y = 0.f, z = 0.f;
 };
 
-// Query row i = e / K of an entry number e < 2^31 without a division
-// instruction: Granlund and Montgomery's method for an invariant unsigned
-// divisor ("Division by invariant integers using multiplication", PLDI
-// 1994): with l = ceil(log2 K) and mul = floor(2^32 (2^l - K) / K) + 1,
-// t = umulhi(mul, e) and e / K = (t + ((e - t) >> min(l, 1))) >> max(l - 1, 0).
-struct DivK {
-  uint32_t mul;
-  int s1, s2;
-};
-
-DivK make_divk(uint32_t d) {
-  int l = 0;
-  while ((1ull << l) < d) ++l;
-  DivK r;
-  r.mul = static_cast<uint32_t>(((1ull << 32) * ((1ull << l) - d)) / d + 1);
-  r.s1 = l < 1 ? l : 1;
-  r.s2 = l > 1 ? l - 1 : 0;
-  return r;
-}
-
-__device__ __forceinline__ uint32_t div_k(uint32_t e, const DivK& dk) {
-  const uint32_t t = __umulhi(dk.mul, e);
-  return (t + ((e - t) >> dk.s1)) >> dk.s2;
-}
-
 // One term of the reference-side sum, in the order the caller fixes:
 // entry e = i*K+j adds -2 g_e (q_i - p).
 __device__ __forceinline__ void add_entry(Acc& a, uint32_t e, const float* __restrict__ q_xyz,
-                                          const float* __restrict__ grad, const DivK& k, float px,
+                                          const float* __restrict__ grad, const FastDiv& k, float px,
                                           float py, float pz) {
-  const int64_t i = div_k(e, k);
+  const int64_t i = fast_div(e, k);
   const float g2 = __fmul_rn(-2.f, grad[e]);
   a.x = __fmaf_rn(g2, __fsub_rn(q_xyz[3 * i], px), a.x);
   a.y = __fmaf_rn(g2, __fsub_rn(q_xyz[3 * i + 1], py), a.y);
@@ -200,7 +175,7 @@ __device__ __forceinline__ void add_entry(Acc& a, uint32_t e, const float* __res
 template <int CAP>
 __device__ __forceinline__ void sum_short(Acc& a, const uint32_t* __restrict__ seg, uint32_t len,
                                           const float* __restrict__ q_xyz,
-                                          const float* __restrict__ grad, const DivK& k, float px,
+                                          const float* __restrict__ grad, const FastDiv& k, float px,
                                           float py, float pz) {
   uint32_t L[CAP];
 #pragma unroll
@@ -220,7 +195,7 @@ __device__ __forceinline__ void sum_short(Acc& a, const uint32_t* __restrict__ s
 // so the order and the arithmetic are those of the short path.
 __global__ void __maxnreg__(96)
     k_bwd_support(const float* __restrict__ q_xyz, const float* __restrict__ p_xyz, int64_t n,
-                  DivK k, const uint32_t* __restrict__ start, const uint32_t* __restrict__ seg,
+                  FastDiv k, const uint32_t* __restrict__ start, const uint32_t* __restrict__ seg,
                   const float* __restrict__ grad, float* __restrict__ grad_p, int accumulate) {
   chain_wait();
   const int64_t p0 = static_cast<int64_t>(blockIdx.x) * blockDim.x;
@@ -358,7 +333,7 @@ int run_backward(const BackwardArgs& a, void* ws, size_t ws_bytes, cudaStream_t 
       ++nl;
     }
     launch_chained(k_bwd_support, blocks_for(a.n, 128), 128, 0, s, a.q_xyz, a.p_xyz, a.n,
-                   make_divk(static_cast<uint32_t>(a.k)), b.start, b.seg, a.grad, a.grad_p,
+                   make_fast_div(static_cast<uint32_t>(a.k)), b.start, b.seg, a.grad, a.grad_p,
                    a.accumulate);
     ++nl;
   }

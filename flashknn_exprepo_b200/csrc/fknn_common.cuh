@@ -164,6 +164,32 @@ __device__ __forceinline__ void copy_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// ------------------------------------------------- division by a constant
+// e / d of an e < 2^31 without a division instruction: Granlund and
+// Montgomery's method for an invariant unsigned divisor ("Division by
+// invariant integers using multiplication", PLDI 1994): with
+// l = ceil(log2 d) and mul = floor(2^32 (2^l - d) / d) + 1,
+// t = umulhi(mul, e) and e / d = (t + ((e - t) >> min(l, 1))) >> max(l - 1, 0).
+struct FastDiv {
+  uint32_t mul;
+  int s1, s2;
+};
+
+inline FastDiv make_fast_div(uint32_t d) {
+  int l = 0;
+  while ((1ull << l) < d) ++l;
+  FastDiv r;
+  r.mul = static_cast<uint32_t>(((1ull << 32) * ((1ull << l) - d)) / d + 1);
+  r.s1 = l < 1 ? l : 1;
+  r.s2 = l > 1 ? l - 1 : 0;
+  return r;
+}
+
+__device__ __forceinline__ uint32_t fast_div(uint32_t e, const FastDiv& d) {
+  const uint32_t t = __umulhi(d.mul, e);
+  return (t + ((e - t) >> d.s1)) >> d.s2;
+}
+
 // ------------------------------------------------------ warp primitives
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;

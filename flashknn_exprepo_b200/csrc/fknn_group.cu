@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Any width and alignment: one warp per row, one word per lane.
+// Any alignment: one warp per row, one word per lane.
 __global__ void __launch_bounds__(256)
     kg_forward_rows(const float* __restrict__ feat, int64_t n, int c,
                     const int32_t* __restrict__ idx, int64_t rows, int k,
@@ -173,6 +173,39 @@ __global__ void __launch_bounds__(256)
       }
       __stcs(out + r * cw + col, v);
     }
+  }
+}
+
+// Narrow rows, flat over the output: thread t writes words t, t + threads, ...,
+// so a warp's stores are one run and neighbouring lanes read one feature row.
+// words < 2^31 (the caller launches slabs of rows); the row and the query each
+// come from a multiplication (fast_div).  A row of one word or a few leaves
+// most lanes of the two kernels above idle: 1.6 million rows took 111 us with
+// one channel and 113 us with six, this takes 13 and 25 us.
+__global__ void __launch_bounds__(256)
+    kg_forward_words(const float* __restrict__ feat, int64_t n, int c,
+                     const int32_t* __restrict__ idx, uint32_t words, FastDiv by_width,
+                     uint32_t row0, FastDiv by_k, const float* __restrict__ xyz,
+                     const float* __restrict__ new_xyz, int off, float* __restrict__ out,
+                     int* status) {
+  chain_wait();
+  const uint32_t cw = static_cast<uint32_t>(c + off);
+  const uint32_t stride = gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += stride) {
+    const uint32_t r = fast_div(w, by_width);
+    const int col = static_cast<int>(w - r * cw);
+    const int32_t t = __ldg(idx + r);
+    float v = 0.f;
+    if (entry_ok(t, n, col == 0 ? status : nullptr)) {
+      if (col >= off) {
+        v = __ldg(feat + static_cast<int64_t>(t) * c + (col - off));
+      } else {
+        const int64_t i = fast_div(row0 + r, by_k);
+        v = __fsub_rn(__ldg(xyz + 3 * static_cast<int64_t>(t) + col), __ldg(new_xyz + 3 * i + col));
+      }
+    }
+    __stcs(out + w, v);
   }
 }
 
@@ -438,16 +471,37 @@ int run_group_forward(const GroupArgs& g, void* ws, size_t ws_bytes, cudaStream_
     // within 40 KB (five CTAs per SM), 4 up to the 48 KB that need no opt-in;
     // wider rows amortise the per-row work by themselves.
     const int R = cw <= 160 ? 8 : (cw <= 384 ? 4 : 0);
+    // Staged runs pay where a feature row fills a good part of a warp's loads
+    // and there are enough rows for its warps.  Float4 features from 16
+    // channels up: with xyz, 1.6 million rows take 66 us (word by word 74) at
+    // 16 channels, but 60 (46) at 8.  Other features from 57 up: 960 thousand
+    // rows take 105 us (word by word 111) at 57 channels and 111 (97) at 49.
+    // Fewer rows leave warps without a run, and each run is a longer chain of
+    // loads: 960 rows of 3 + 16 take 6.4 us (4.6 word by word), 16 thousand
+    // rows of 3 + 97 take 14.1 us (8.5 by warps of one row).
+    const bool wide = g.c > 56;
+    const bool staged = out16 && R && (feat4 ? g.c >= 16 && rows >= 4096 : wide && rows >= 65536);
     if (feat4 && out16 && !off) {
       launch_chained(kg_forward, capped_blocks(rows * tpr), 256, 0, s, g.feat, g.n, g.c, g.idx,
                      rows, tpr, g.out, &b.meta->status);
-    } else if (out16 && R && rows <= INT32_MAX) {
+    } else if (staged) {
       launch_chained(kg_forward_staged, capped_warp_blocks(ceil_div(rows, R)), 256,
                      sizeof(float) * 8 * R * cw, s, g.feat, g.n, g.c, g.idx, rows, g.k, g.xyz,
                      g.new_xyz, off, R, tpr, g.out, &b.meta->status);
-    } else {
+    } else if (wide) {
       launch_chained(kg_forward_rows, capped_warp_blocks(rows), 256, 0, s, g.feat, g.n, g.c, g.idx,
                      rows, g.k, g.xyz, g.new_xyz, off, g.out, &b.meta->status);
+    } else {
+      const int64_t slab = INT32_MAX / cw;  // rows per launch
+      for (int64_t r0 = 0; r0 < rows; r0 += slab) {
+        const int64_t words = (rows - r0 < slab ? rows - r0 : slab) * cw;
+        if (r0 > 0) ++nl;
+        launch_chained(kg_forward_words, capped_blocks(words), 256, 0, s, g.feat, g.n, g.c,
+                       g.idx + r0, static_cast<uint32_t>(words),
+                       make_fast_div(static_cast<uint32_t>(cw)), static_cast<uint32_t>(r0),
+                       make_fast_div(static_cast<uint32_t>(g.k)), g.xyz, g.new_xyz, off,
+                       g.out + r0 * cw, &b.meta->status);
+      }
     }
     ++nl;
   }

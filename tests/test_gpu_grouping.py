@@ -129,3 +129,44 @@ def test_row_widths_and_alignments(fk, m, k, c, shift, with_xyz):
     got = {"feat": feat.grad, "xyz": xyz.grad, "new_xyz": new.grad}
     for key in ("feat",) + (("xyz", "new_xyz") if with_xyz else ()):
         assert rel(got[key].cpu().numpy(), want[key]) <= 1e-5
+
+
+@pytest.mark.parametrize("with_xyz", [False, True])
+@pytest.mark.parametrize("m,k", [(1365, 3), (256, 16), (8192, 8), (65535, 1)])
+@pytest.mark.parametrize("c,shift", [(12, 0), (16, 0), (16, 1), (56, 0), (57, 0), (57, 1), (157, 0),
+                                     (160, 0), (381, 0), (384, 0), (385, 0)])
+def test_gather_paths_by_width_and_rows(fk, m, k, c, shift, with_xyz):
+    """The gather's paths on both sides of their lines (16 channels and 4,096
+    rows, 57 channels and 65,536 rows, runs of 8 and 4 rows, none)."""
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(c + m)
+    n = 1000
+    idx = torch.randint(-1, n, (m, k), generator=gen, device=DEV, dtype=torch.int32)
+    feat = torch.randn(n * c + shift, generator=gen, device=DEV)[shift:].view(n, c)
+    xyz = torch.rand((n, 3), generator=gen, device=DEV)
+    new = torch.rand((m, 3), generator=gen, device=DEV)
+    il = idx.long()
+    want = feat[il]
+    if with_xyz:
+        want = torch.cat([xyz[il] - new[:, None, :], want], -1)
+    want = torch.where((il >= 0)[..., None], want, torch.zeros_like(want))
+    got = fk.ops.group_features(feat, idx, xyz, new, with_xyz=with_xyz, validate=True)
+    assert torch.equal(got, want)
+
+
+def test_gather_of_more_than_2_31_words(fk):
+    """Narrow rows are gathered in slabs of fewer than 2^31 words: the rows
+    around the line between two slabs, inside one query's run, and the last."""
+    m, k, c, n = 14_000_001, 3, 50, 997
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(3)
+    idx = torch.randint(-1, n, (m, k), generator=gen, device=DEV, dtype=torch.int32)
+    feat = torch.randn((n, c), generator=gen, device=DEV)
+    xyz = torch.rand((n, 3), generator=gen, device=DEV)
+    new = torch.rand((m, 3), generator=gen, device=DEV)
+    out = fk.ops.group_features(feat, idx, xyz, new, with_xyz=True, validate=True)
+    line = (2 ** 31 - 1) // (c + 3) // k
+    for q in (slice(0, 1000), slice(line - 1000, line + 1000), slice(m - 1000, m)):
+        il = idx[q].long()
+        want = torch.cat([xyz[il] - new[q, None, :], feat[il]], -1)
+        assert torch.equal(out[q], torch.where((il >= 0)[..., None], want, torch.zeros_like(want)))
