@@ -269,20 +269,24 @@ struct Vec<2> {
 // One warp per support point: its entries in ascending order, each row of
 // grad_out added channel by channel in that order.  V channels per lane (2
 // when the rows are whole float2s) and NC column blocks of 32*V channels, so
-// rows of up to 32*V*NC channels are read in one walk over the entries; the
-// rows of kRows entries are loaded before they are added, in order, so
-// kRows*NC loads are in flight per lane.  Bound by reading grad_out once: walking the
-// entries again for every 32 channels (NC = 1), 3.2 million rows of 3 + 64
-// floats (858 MB) took 321 us, one walk with four
-// rows in flight 296 us, with eight 218 us.
+// rows of up to 32*V*NC channels are read in one walk over the entries.  Bound
+// by reading grad_out once, at random rows.  Rows of several blocks: the rows
+// of eight entries are loaded before they are added, in order, so 8*NC loads
+// are in flight per lane; walking the entries again for every 32 channels,
+// 3.2 million rows of 3 + 64 floats (858 MB) took 321 us, one walk with four
+// rows in flight 296 us, with eight 218 us.  Rows of one block keep few loads
+// in flight whatever the unroll, so warps count instead: four rows at a time
+// in 32 registers (eight CTAs per SM).  The whole backward of 1.6 million
+// rows, segments of 16, takes 90 us with 2 channels (eight rows in 63
+// registers: 115) and 133 us with 64 (150).
 template <int V, int NC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, NC == 1 ? 8 : (V == 1 ? 4 : 3))
     kg_support(const float* __restrict__ grad_out, int c, int with_xyz,
                const uint32_t* __restrict__ start, const uint32_t* __restrict__ seg, int64_t n,
                float* __restrict__ grad_feat, float* __restrict__ grad_xyz, int accumulate_xyz) {
   chain_wait();
   using VT = typename Vec<V>::T;
-  constexpr int kRows = 8;
+  constexpr int kRows = 8, kAhead = 8;
   const int lane = threadIdx.x & 31;
   const int off = with_xyz ? 3 : 0;
   const int cw = c + off;
@@ -310,7 +314,27 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int b = 0; b < NC; ++b) acc[b] = Vec<V>::add(acc[b], v[b]);
       };
-      if (len <= 32) {
+      if (len <= 32 && NC == 1) {
+        const int col = c0 + lane * V;
+        const bool live = col < cw;
+        const float* at = grad_out + col;
+        auto row = [&](uint32_t e) {
+          return *reinterpret_cast<const VT*>(at + static_cast<int64_t>(e) * cw);
+        };
+        uint32_t r = 0;
+        for (; r + 4 <= len; r += 4) {
+          const uint32_t e0 = __shfl_sync(kFull, mine, r), e1 = __shfl_sync(kFull, mine, r + 1);
+          const uint32_t e2 = __shfl_sync(kFull, mine, r + 2), e3 = __shfl_sync(kFull, mine, r + 3);
+          if (live) {
+            const VT v0 = row(e0), v1 = row(e1), v2 = row(e2), v3 = row(e3);
+            acc[0] = Vec<V>::add(Vec<V>::add(Vec<V>::add(Vec<V>::add(acc[0], v0), v1), v2), v3);
+          }
+        }
+        for (; r < len; ++r) {
+          const uint32_t e = __shfl_sync(kFull, mine, r);
+          if (live) acc[0] = Vec<V>::add(acc[0], row(e));
+        }
+      } else if (len <= 32) {
         for (uint32_t r = 0; r < len; r += kRows) {
           VT v[kRows][NC];
 #pragma unroll
@@ -321,18 +345,40 @@ __global__ void __launch_bounds__(256)
             if (r + u < len) add(v[u]);
         }
       } else {
-        uint32_t last = 0;
-        for (uint32_t r = 0; r < len; ++r) {
-          uint32_t best = kNoEntry;
-          for (uint32_t t = lane; t < len; t += 32) {
-            const uint32_t v = seg[s + t];
-            if ((r == 0 || v > last) && v < best) best = v;
+        // The two smallest entries from `next` on, per pass over the segment:
+        // as unsigned differences the ones before it wrap to above every entry
+        // (entries are below 2^31).  Bound by the passes' loads (latency):
+        // kAhead at a time, the backward of 800 thousand entries on 64 points
+        // takes 68 ms with 3 channels, one entry a pass and one load at a time
+        // 715 ms.
+        uint32_t next = 0;
+        for (uint32_t r = 0; r < len; r += 2) {
+          uint32_t g0 = kNoEntry, g1 = kNoEntry, t = lane;
+          const uint32_t* at = seg + s + lane;
+          auto take = [&](uint32_t v) {
+            g1 = min(g1, max(g0, v));
+            g0 = min(g0, v);
+          };
+#pragma unroll 1
+          for (; t + 32 * (kAhead - 1) < len; t += 32 * kAhead, at += 32 * kAhead) {
+            uint32_t v[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) v[u] = __ldg(at + 32 * u);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) take(v[u] - next);
           }
-          best = __reduce_min_sync(kFull, best);
+#pragma unroll 1
+          for (; t < len; t += 32, at += 32) take(__ldg(at) - next);
+          const uint32_t first = __reduce_min_sync(kFull, g0);
+          const uint32_t second = __reduce_min_sync(kFull, g0 == first ? g1 : g0);
           VT v[NC];
-          load(best, v);
+          load(next + first, v);
           add(v);
-          last = best;
+          if (r + 1 < len) {
+            load(next + second, v);
+            add(v);
+          }
+          next += second + 1;
         }
       }
 #pragma unroll

@@ -170,3 +170,29 @@ def test_gather_of_more_than_2_31_words(fk):
         il = idx[q].long()
         want = torch.cat([xyz[il] - new[q, None, :], feat[il]], -1)
         assert torch.equal(out[q], torch.where((il >= 0)[..., None], want, torch.zeros_like(want)))
+
+
+@pytest.mark.parametrize("c,with_xyz", [(3, False), (16, False), (29, True), (64, False),
+                                        (61, True), (100, False), (93, True), (131, False)])
+def test_backward_adds_rows_in_entry_order(fk, c, with_xyz):
+    """Segment lengths on both sides of a warp's 32 entries and of the long
+    segments' passes (two entries each, 256 loaded at a time), odd and even,
+    every column split: the FP32 sums in ascending entry order, bit for bit."""
+    lens = [0, 1, 3, 4, 5, 7, 8, 9, 31, 32, 33, 34, 63, 64, 65, 224, 225, 255, 256, 257, 300, 513]
+    rng = np.random.default_rng(c)
+    idx = np.concatenate([np.full(q, t, np.int32) for t, q in enumerate(lens)] +
+                         [np.full(40, -1, np.int32)])
+    rng.shuffle(idx)
+    off = 3 if with_xyz else 0
+    grad = rng.standard_normal((len(idx), 1, c + off)).astype(np.float32)
+    want = np.zeros((len(lens), c + off), np.float32)
+    for e, t in enumerate(idx):
+        if t >= 0:
+            want[t] += grad[e, 0]
+    n = len(lens)
+    feat = torch.empty((n, c), device=DEV)
+    xyz = torch.empty((n, 3), device=DEV) if with_xyz else None
+    fk.ops.group_backward(T(grad), T(idx[:, None]), n, c, with_xyz, feat, xyz)
+    assert np.array_equal(feat.cpu().numpy(), want[:, off:])
+    if with_xyz:
+        assert np.array_equal(xyz.cpu().numpy(), want[:, :3])
