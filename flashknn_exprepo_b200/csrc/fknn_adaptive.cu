@@ -797,8 +797,7 @@ int run_adaptive(const AdaptiveArgs& f, void* ws, size_t ws_bytes, const QuerySh
     ++nl;
   }
   nl += launch_items(b.runs, b.group_start, b.group_start + 1, b.group_row, &b.meta->n_groups, n,
-                     shape.tile_records, b.cands, &b.meta->n_items, b.items, s, &b.meta->status, n,
-                     false);
+                     shape.tile_records, b.cands, b.meta, b.items, s, n, false);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     note_cuda_error(e);

@@ -489,18 +489,20 @@ __device__ __forceinline__ int2 hash_find(const HashSlot* table, uint32_t mask, 
 // key in the support key space; runs[g*27 + j] = (start, count) of the
 // support cell at offset j, or (0, 0) when that cell is empty.  With cands,
 // cands[g] = the group's candidate total (the work-item packer's input; a
-// group without candidates sets kStatusNoCandidates in *status) and
-// meta->cand_total receives the sum of the totals (one atomic per block).
+// group without candidates sets kStatusNoCandidates in *status), and
+// meta->cand_total and pair_total receive the sums of the totals and of the
+// totals times the group's queries (one atomic each per block).
 __global__ void __launch_bounds__(256)
     k_runs(const uint64_t* __restrict__ group_key, const int* group_count_ptr,
            const HashSlot* __restrict__ table, uint32_t hmask, const int* cell_count_ptr,
            Meta* meta, int2* __restrict__ runs, int32_t* __restrict__ cands,
+           const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
            int* status) {
   chain_wait();
-  __shared__ unsigned long long block_total;
-  if (threadIdx.x == 0) block_total = 0ull;
+  __shared__ unsigned long long block_total, block_pairs;
+  if (threadIdx.x == 0) block_total = block_pairs = 0ull;
   __syncthreads();
-  unsigned long long my_total = 0ull;
+  unsigned long long my_total = 0ull, my_pairs = 0ull;
   const int groups = *group_count_ptr;
   const int bpa = meta->bpa;
   const int cells = *cell_count_ptr;
@@ -531,14 +533,21 @@ __global__ void __launch_bounds__(256)
       if (j == 0) {
         cands[g] = total;
         my_total += static_cast<unsigned long long>(total);
+        my_pairs += static_cast<unsigned long long>(total) * (group_end[g] - group_start[g]);
         if (total == 0) raise_status(status, kStatusNoCandidates);
       }
     }
   }
   if (cands) {
-    if (my_total) atomicAdd(&block_total, my_total);
+    if (my_total) {
+      atomicAdd(&block_total, my_total);
+      atomicAdd(&block_pairs, my_pairs);
+    }
     __syncthreads();
-    if (threadIdx.x == 0 && block_total) atomicAdd(&meta->cand_total, block_total);
+    if (threadIdx.x == 0 && block_total) {
+      atomicAdd(&meta->cand_total, block_total);
+      atomicAdd(&meta->pair_total, block_pairs);
+    }
   }
 }
 
@@ -859,11 +868,10 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     if (n > 0) {
       launch_chained(k_runs, capped_blocks(n * 32), 256, 0, s, b.cell_key, &b.meta->n_cells,
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
-                     &b.meta->status);
+                     b.cell_start, b.cell_end, &b.meta->status);
       ++nl;
       nl += launch_items(b.runs, b.cell_start, b.cell_end, nullptr, &b.meta->n_cells, n,
-                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
-                         &b.meta->status, n, true);
+                         shape.tile_records, b.cands, b.meta, b.items, s, n, true);
     }
   } else if (kind == FKNN_QUERY_SELECTED) {
     pad_mode = kPadArray64;
@@ -876,7 +884,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     group_count_ptr = &b.meta->n_groups;
     if (n > 0) {
       launch_chained(k_runs, capped_blocks(n * 32), 256, 0, s, b.cell_key,
-          &b.meta->n_cells, b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, nullptr, nullptr);
+          &b.meta->n_cells, b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, nullptr, nullptr, nullptr, nullptr);
       ++nl;
     }
     if (m > 0 && n > 0) {
@@ -897,8 +905,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
           b.srec, b.slot_of, b.rank_of, b.qstart, b.qrec, &b.meta->status);
       nl += 6;
       nl += launch_items(b.runs, b.group_start, group_end, b.group_row, &b.meta->n_groups, m,
-                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
-                         &b.meta->status, m, false);
+                         shape.tile_records, b.cands, b.meta, b.items, s, m, false);
     }
   } else {  // general queries
     pad_mode = kPadMinusOne;
@@ -924,11 +931,10 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
       nl += 3;
       launch_chained(k_runs, capped_blocks(m * 32), 256, 0, s, b.group_key, &b.meta->n_groups,
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
-                     &b.meta->status);
+                     b.group_start, b.group_end, &b.meta->status);
       ++nl;
       nl += launch_items(b.runs, b.group_start, b.group_end, nullptr, &b.meta->n_groups, m,
-                         shape.tile_records, b.cands, &b.meta->n_items, b.items, s,
-                         &b.meta->status, m, true);
+                         shape.tile_records, b.cands, b.meta, b.items, s, m, true);
     }
   }
 

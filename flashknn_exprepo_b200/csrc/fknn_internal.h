@@ -34,8 +34,10 @@ struct Meta {
   // sum over the query groups of their 27-cell candidate totals (self and
   // general queries; read back for FlashKNN.query's traverse_info)
   unsigned long long cand_total;
+  // sum over the query groups of queries x candidates (chunked item sizes)
+  unsigned long long pair_total;
 };
-static_assert(sizeof(Meta) == 64, "Meta layout");
+static_assert(sizeof(Meta) == 72, "Meta layout");
 static_assert(offsetof(Meta, cand_total) == 56, "Meta layout");
 
 // Work items (int4): (q_start, q_count, g_first, g_count | flags) -- the
@@ -86,12 +88,13 @@ struct QueryLaunch {
 int launch_query(const QueryLaunch& q, const QueryShape& shape, cudaStream_t s);
 
 // Item construction (fknn_items.cu): per-group candidate counts, segmented
-// greedy packing; *n_items_ptr (0 before) receives the item count.  Group g's
-// queries are the records [group_start[g], group_end[g]).  Returns launches.
+// greedy packing; meta->n_items (0 before) receives the item count.  Group g's
+// queries are the records [group_start[g], group_end[g]).  cands_ready: cands
+// and meta->pair_total (0 before) are there already.  Returns launches.
 int launch_items(const int2* runs, const int32_t* group_start, const int32_t* group_end,
                  const int32_t* group_row, const int* group_count_ptr, int64_t max_groups, int tile,
-                 int32_t* cands, int* n_items_ptr, int4* items, cudaStream_t s, int* status,
-                 int64_t n_queries, bool cands_ready);
+                 int32_t* cands, Meta* meta, int4* items, cudaStream_t s, int64_t n_queries,
+                 bool cands_ready);
 size_t items_capacity(int64_t max_groups, int64_t n_queries);
 // Bounded-wait self-test (fknn_selftest.cu): arms a barrier that never
 // completes and waits at most `limit` polls; sets kStatusTimeout.

@@ -24,11 +24,18 @@
 namespace fknn {
 
 // cands[g] = number of candidate records of group g (sum of its 27 runs);
-// a group without candidates sets kStatusNoCandidates when status is given.
+// a group without candidates sets kStatusNoCandidates.  meta->pair_total
+// receives the sum of queries x candidates (one atomic per block).
 __global__ void __launch_bounds__(256)
     k_group_cands(const int2* __restrict__ runs, const int32_t* __restrict__ group_row,
-                  const int* group_count_ptr, int32_t* __restrict__ cands, int* status) {
+                  const int* group_count_ptr, int32_t* __restrict__ cands,
+                  const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
+                  Meta* meta) {
   chain_wait();
+  __shared__ unsigned long long block_pairs;
+  if (threadIdx.x == 0) block_pairs = 0ull;
+  __syncthreads();
+  unsigned long long my_pairs = 0ull;
   const int n_groups = *group_count_ptr;
   for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < n_groups;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -38,24 +45,38 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int j = 0; j < kNeighbours; ++j) total += max(r[j].y, 0);
     cands[g] = total;
-    if (total == 0) raise_status(status, kStatusNoCandidates);
+    my_pairs += static_cast<unsigned long long>(total) * max(group_end[g] - group_start[g], 0);
+    if (total == 0) raise_status(&meta->status, kStatusNoCandidates);
   }
+  if (my_pairs) atomicAdd(&block_pairs, my_pairs);
+  __syncthreads();
+  if (threadIdx.x == 0 && block_pairs) atomicAdd(&meta->pair_total, block_pairs);
 }
 
-// Queries of a chunked item of a group with c candidates.  In a large problem
-// (max_qc = 32) max_qc up to kChunkedFull candidates, then fewer in inverse
-// proportion, at least kChunkedFew: an item's time grows with c, and with full
-// items the heaviest ones (13 thousand candidates) ran on for twice the mean
-// after the others had ended.  A LiDAR scan with 40 cm cells (115 thousand
-// queries) takes 325 us at K=16 and 547 us at K=32, with full items 480 and
-// 728 us; from 1,024 candidates on, or down to 4 queries, it is slower (329 to
-// 382 and 549 to 661 us).  A smaller problem is cut to two items per warp
-// already (chunked_query_cap) and keeps that size: cut further, the DeLA
-// levels gained nothing.
+// Queries of a chunked item of a group with c candidates.  Below a full
+// item's worth of queries per resident warp (max_qc < 32, chunked_query_cap)
+// max_qc.  In a larger problem an item's time grows with c, and smaller items
+// stream the candidates more often, so an item is cut only where it would
+// run on after the others have ended.  `share` = candidates that an average
+// lane meets in the whole call (pairs of query and candidate over the resident
+// lanes): a full item of c = share keeps its warp busy for the average warp's
+// whole time.  Groups of usual size (c up to 3/2 of the mean over the queries)
+// carry most of the work and are cut to that time; groups far above it to a
+// quarter, since a few of them decide when the call ends.  Never below
+// kChunkedFull candidates or to fewer than kChunkedFew queries.  K=16, whole
+// call, full items / every group above 2,048 candidates cut in inverse
+// proportion / this rule: a LiDAR scan of 115 thousand points with 40 cm cells
+// (up to 13 thousand candidates) 404 / 282 / 277 us, one of 800 thousand 2993 /
+// 3168 / 2481; 500 thousand uniform points of 20 thousand candidates 2511 /
+// 3248 / 1940, 400 thousand on a sheet of 12 thousand 2070 / 2749 / 1571 (the
+// first figure with an earlier scan kernel, 1.3 times slower by itself).  One
+// limit for all groups: half a share 5 to 12 % slower on scans of 400
+// thousand, a quarter up to 15 % on uniform points.
 constexpr int kChunkedFull = 2048, kChunkedFew = 8;
-__device__ __forceinline__ int chunked_queries(int max_qc, int c) {
-  if (c <= kChunkedFull || max_qc < 32) return max_qc;
-  return max(static_cast<int>(static_cast<int64_t>(max_qc) * kChunkedFull / c), kChunkedFew);
+__device__ __forceinline__ int chunked_queries(int max_qc, int c, int64_t typical, int64_t share) {
+  const int64_t full = max(c <= typical ? share : share / 4, static_cast<int64_t>(kChunkedFull));
+  if (c <= full || max_qc < 32) return max_qc;
+  return max(static_cast<int>(max_qc * full / c), kChunkedFew);
 }
 
 // One warp per segment of consecutive groups.  Item = (q_start, q_count,
@@ -74,9 +95,14 @@ static_assert(kPackSegment <= 32, "one group per lane");
 __global__ void __launch_bounds__(256)
     k_pack(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
            const int32_t* __restrict__ cands, const int* group_count_ptr, int tile, int max_q,
-           int max_qc, int64_t n_queries, int64_t capacity, int* n_items, int4* __restrict__ items,
-           int* status) {
+           int max_qc, int64_t n_queries, int64_t capacity, int64_t lanes, Meta* meta,
+           int4* __restrict__ items) {
   chain_wait();
+  int* n_items = &meta->n_items;
+  int* status = &meta->status;
+  const double pairs = static_cast<double>(meta->pair_total);
+  const int64_t typical = static_cast<int64_t>(1.5 * pairs / static_cast<double>(n_queries));
+  const int64_t share = static_cast<int64_t>(pairs / static_cast<double>(lanes));
   __shared__ uint32_t s_count[8];
   __shared__ uint32_t s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -124,7 +150,7 @@ __global__ void __launch_bounds__(256)
         if (ge <= gs) continue;
         if (c > tile) {  // streams its candidates: items of its own
           flush();
-          const int qc = chunked_queries(max_qc, c);
+          const int qc = chunked_queries(max_qc, c, typical, share);
           const int n_it = (ge - gs + qc - 1) / qc;
           if (write)
             for (int t = lane; t < n_it; t += 32) {
@@ -192,29 +218,33 @@ int item_query_cap(int64_t n_queries) {
   return static_cast<int>(cap < 4 ? 4 : (cap > 32 ? 32 : cap));
 }
 
+// Query warps resident on the current device at the default launch shape; 0
+// where the device does not tell.
+int64_t resident_warps() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return 0;
+  return static_cast<int64_t>(sms) * 20;
+}
+
 // Queries per chunked item (a group whose candidates exceed a tile: every
 // query scans many of them).  An item of q queries gives each query 32 / q
 // lanes.  A problem with fewer than 32 queries per resident query warp is
 // cut into about two items per warp (at least 4 queries each), so a dense
 // but small problem spreads every query's scan over several lanes instead
-// of one lane walking all its candidates; larger ones keep full items
-// (measured: the LiDAR scan at alpha 8, 118k points, is faster with full
-// items; the DeLA levels of 3.7k-72k points with split ones).
-int chunked_query_cap(int64_t n_queries) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return 32;
-  const int64_t warps = static_cast<int64_t>(sms) * 20;
-  if (n_queries >= warps * 32) return 32;
+// of one lane walking all its candidates (the DeLA levels of 3.7k-72k points
+// are faster so); larger ones start from full items (chunked_queries).
+int chunked_query_cap(int64_t n_queries, int64_t warps) {
+  if (warps == 0 || n_queries >= warps * 32) return 32;
   const int64_t cap = ceil_div(n_queries > 0 ? n_queries : 1, 2 * warps);
   return static_cast<int>(cap < 4 ? 4 : (cap > 32 ? 32 : cap));
 }
 
 int launch_items(const int2* runs, const int32_t* group_start, const int32_t* group_end,
                  const int32_t* group_row, const int* group_count_ptr, int64_t max_groups, int tile,
-                 int32_t* cands, int* n_items_ptr, int4* items, cudaStream_t s, int* status,
-                 int64_t n_queries, bool cands_ready) {
+                 int32_t* cands, Meta* meta, int4* items, cudaStream_t s, int64_t n_queries,
+                 bool cands_ready) {
   if (max_groups <= 0) return 0;
   // grids for the host-side bound, capped: the device count drives the loops
   const int64_t gb = ceil_div(max_groups, 256);
@@ -223,11 +253,12 @@ int launch_items(const int2* runs, const int32_t* group_start, const int32_t* gr
   const int sblocks = static_cast<int>(sb < 2048 ? sb : 2048);
   if (!cands_ready)  // else the caller's run kernel wrote cands[g] already
     launch_chained(k_group_cands, gblocks, 256, 0, s, runs, group_row, group_count_ptr, cands,
-        status);
+                   group_start, group_end, meta);
   const int64_t capacity = static_cast<int64_t>(items_capacity(max_groups, n_queries));
+  const int64_t warps = resident_warps();
   launch_chained(k_pack, sblocks, 256, 0, s, group_start, group_end, cands, group_count_ptr, tile,
-                 item_query_cap(n_queries), chunked_query_cap(n_queries), n_queries, capacity,
-                 n_items_ptr, items, status);
+                 item_query_cap(n_queries), chunked_query_cap(n_queries, warps), n_queries, capacity,
+                 warps > 0 ? warps * 32 : 1, meta, items);
   return cands_ready ? 1 : 2;
 }
 

@@ -175,8 +175,7 @@ int run_tables(const TablesArgs& t, void* ws, size_t ws_bytes, const QueryShape&
   const int32_t* steps = selected ? t.steps_query : t.steps;
   if (t.p > 0)
     nl += launch_items(b.runs, steps, steps + 1, nullptr, &b.meta->n_groups, t.p,
-                       shape.tile_records, b.cands, &b.meta->n_items, b.items, s, &b.meta->status,
-                       selected ? m : t.n, false);
+                       shape.tile_records, b.cands, b.meta, b.items, s, selected ? m : t.n, false);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     note_cuda_error(e);
