@@ -490,18 +490,17 @@ __device__ __forceinline__ int2 hash_find(const HashSlot* table, uint32_t mask, 
 // support cell at offset j, or (0, 0) when that cell is empty.  With cands,
 // cands[g] = the group's candidate total (the work-item packer's input; a
 // group without candidates sets kStatusNoCandidates in *status), and
-// meta->cand_total and pair_total receive the sums of the totals and of the
-// totals times the group's queries (one atomic each per block).
+// meta->cand_total and, with `pairs`, pair_total receive the sums of the totals
+// and of the totals times the group's queries (an atomic each per block).  Without
+// group_end the queries of a group are its centre cell's points.
 __global__ void __launch_bounds__(256)
     k_runs(const uint64_t* __restrict__ group_key, const int* group_count_ptr,
            const HashSlot* __restrict__ table, uint32_t hmask, const int* cell_count_ptr,
            Meta* meta, int2* __restrict__ runs, int32_t* __restrict__ cands,
            const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
-           int* status) {
+           int pairs, int* status) {
   chain_wait();
-  __shared__ unsigned long long block_total, block_pairs;
-  if (threadIdx.x == 0) block_total = block_pairs = 0ull;
-  __syncthreads();
+  __shared__ unsigned long long s_total[8], s_pairs[8];
   unsigned long long my_total = 0ull, my_pairs = 0ull;
   const int groups = *group_count_ptr;
   const int bpa = meta->bpa;
@@ -513,6 +512,8 @@ __global__ void __launch_bounds__(256)
   for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
        g < groups; g += warps) {
     int2 run = make_int2(0, 0);
+    int queries = 0;  // lane 0; in flight during the lookups
+    if (pairs && group_end && j == 0) queries = group_end[g] - group_start[g];
     if (j < kNeighbours) {
       const uint64_t key = group_key[g];
       const uint64_t cloud = key >> (3 * bpa);
@@ -531,22 +532,29 @@ __global__ void __launch_bounds__(256)
     if (cands) {
       const int total = __reduce_add_sync(kFull, run.y);
       if (j == 0) {
+        if (!group_end) queries = run.y;
         cands[g] = total;
         my_total += static_cast<unsigned long long>(total);
-        my_pairs += static_cast<unsigned long long>(total) * (group_end[g] - group_start[g]);
+        my_pairs += static_cast<unsigned long long>(total) * static_cast<unsigned>(queries);
         if (total == 0) raise_status(status, kStatusNoCandidates);
       }
     }
   }
   if (cands) {
-    if (my_total) {
-      atomicAdd(&block_total, my_total);
-      atomicAdd(&block_pairs, my_pairs);
+    if (j == 0) {
+      s_total[threadIdx.x >> 5] = my_total;
+      s_pairs[threadIdx.x >> 5] = my_pairs;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && block_total) {
-      atomicAdd(&meta->cand_total, block_total);
-      atomicAdd(&meta->pair_total, block_pairs);
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) {
+        my_total += s_total[w];
+        my_pairs += s_pairs[w];
+      }
+      if (my_total) {
+        atomicAdd(&meta->cand_total, my_total);
+        if (pairs) atomicAdd(&meta->pair_total, my_pairs);
+      }
     }
   }
 }
@@ -868,7 +876,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     if (n > 0) {
       launch_chained(k_runs, capped_blocks(n * 32), 256, 0, s, b.cell_key, &b.meta->n_cells,
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
-                     b.cell_start, b.cell_end, &b.meta->status);
+                     nullptr, nullptr, pairs_wanted(n) ? 1 : 0, &b.meta->status);
       ++nl;
       nl += launch_items(b.runs, b.cell_start, b.cell_end, nullptr, &b.meta->n_cells, n,
                          shape.tile_records, b.cands, b.meta, b.items, s, n, true);
@@ -884,7 +892,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
     group_count_ptr = &b.meta->n_groups;
     if (n > 0) {
       launch_chained(k_runs, capped_blocks(n * 32), 256, 0, s, b.cell_key,
-          &b.meta->n_cells, b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, nullptr, nullptr, nullptr, nullptr);
+          &b.meta->n_cells, b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, nullptr, nullptr, nullptr, 0, nullptr);
       ++nl;
     }
     if (m > 0 && n > 0) {
@@ -931,7 +939,7 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
       nl += 3;
       launch_chained(k_runs, capped_blocks(m * 32), 256, 0, s, b.group_key, &b.meta->n_groups,
                      b.hslots, hmask, &b.meta->n_cells, b.meta, b.runs, b.cands,
-                     b.group_start, b.group_end, &b.meta->status);
+                     b.group_start, b.group_end, pairs_wanted(m) ? 1 : 0, &b.meta->status);
       ++nl;
       nl += launch_items(b.runs, b.group_start, b.group_end, nullptr, &b.meta->n_groups, m,
                          shape.tile_records, b.cands, b.meta, b.items, s, m, true);

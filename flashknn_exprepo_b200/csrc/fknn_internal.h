@@ -90,12 +90,14 @@ int launch_query(const QueryLaunch& q, const QueryShape& shape, cudaStream_t s);
 // Item construction (fknn_items.cu): per-group candidate counts, segmented
 // greedy packing; meta->n_items (0 before) receives the item count.  Group g's
 // queries are the records [group_start[g], group_end[g]).  cands_ready: cands
-// and meta->pair_total (0 before) are there already.  Returns launches.
+// and, where pairs_wanted, meta->pair_total (0 before) are there already.
+// Returns launches.
 int launch_items(const int2* runs, const int32_t* group_start, const int32_t* group_end,
                  const int32_t* group_row, const int* group_count_ptr, int64_t max_groups, int tile,
                  int32_t* cands, Meta* meta, int4* items, cudaStream_t s, int64_t n_queries,
                  bool cands_ready);
 size_t items_capacity(int64_t max_groups, int64_t n_queries);
+bool pairs_wanted(int64_t n_queries);
 // Bounded-wait self-test (fknn_selftest.cu): arms a barrier that never
 // completes and waits at most `limit` polls; sets kStatusTimeout.
 int run_selftest_wait(void* ws, size_t ws_bytes, uint32_t limit, cudaStream_t s);

@@ -25,16 +25,15 @@ namespace fknn {
 
 // cands[g] = number of candidate records of group g (sum of its 27 runs);
 // a group without candidates sets kStatusNoCandidates.  meta->pair_total
-// receives the sum of queries x candidates (one atomic per block).
+// receives the sum of queries x candidates (one atomic per block)
+// where it is wanted (pairs_wanted).
 __global__ void __launch_bounds__(256)
     k_group_cands(const int2* __restrict__ runs, const int32_t* __restrict__ group_row,
                   const int* group_count_ptr, int32_t* __restrict__ cands,
                   const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
-                  Meta* meta) {
+                  int pairs, Meta* meta) {
   chain_wait();
-  __shared__ unsigned long long block_pairs;
-  if (threadIdx.x == 0) block_pairs = 0ull;
-  __syncthreads();
+  __shared__ unsigned long long s_pairs[8];
   unsigned long long my_pairs = 0ull;
   const int n_groups = *group_count_ptr;
   for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < n_groups;
@@ -45,12 +44,19 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int j = 0; j < kNeighbours; ++j) total += max(r[j].y, 0);
     cands[g] = total;
-    my_pairs += static_cast<unsigned long long>(total) * max(group_end[g] - group_start[g], 0);
+    if (pairs)
+      my_pairs += static_cast<unsigned long long>(total) * max(group_end[g] - group_start[g], 0);
     if (total == 0) raise_status(&meta->status, kStatusNoCandidates);
   }
-  if (my_pairs) atomicAdd(&block_pairs, my_pairs);
+  if (!pairs) return;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) my_pairs += __shfl_xor_sync(kFull, my_pairs, d);
+  if ((threadIdx.x & 31) == 0) s_pairs[threadIdx.x >> 5] = my_pairs;
   __syncthreads();
-  if (threadIdx.x == 0 && block_pairs) atomicAdd(&meta->pair_total, block_pairs);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) my_pairs += s_pairs[w];
+    if (my_pairs) atomicAdd(&meta->pair_total, my_pairs);
+  }
 }
 
 // Queries of a chunked item of a group with c candidates.  Below a full
@@ -72,11 +78,13 @@ __global__ void __launch_bounds__(256)
 // first figure with an earlier scan kernel, 1.3 times slower by itself).  One
 // limit for all groups: half a share 5 to 12 % slower on scans of 400
 // thousand, a quarter up to 15 % on uniform points.
-constexpr int kChunkedFull = 2048, kChunkedFew = 8;
-__device__ __forceinline__ int chunked_queries(int max_qc, int c, int64_t typical, int64_t share) {
-  const int64_t full = max(c <= typical ? share : share / 4, static_cast<int64_t>(kChunkedFull));
-  if (c <= full || max_qc < 32) return max_qc;
-  return max(static_cast<int>(max_qc * full / c), kChunkedFew);
+constexpr float kChunkedFull = 2048.f;
+constexpr int kChunkedFew = 8;
+__device__ __forceinline__ int chunked_queries(int max_qc, int c, float typical, float share) {
+  const float cf = static_cast<float>(c);
+  const float full = fmaxf(cf <= typical ? share : 0.25f * share, kChunkedFull);
+  if (cf <= full || max_qc < 32) return max_qc;
+  return max(static_cast<int>(static_cast<float>(max_qc) * full / cf), kChunkedFew);
 }
 
 // One warp per segment of consecutive groups.  Item = (q_start, q_count,
@@ -95,14 +103,13 @@ static_assert(kPackSegment <= 32, "one group per lane");
 __global__ void __launch_bounds__(256)
     k_pack(const int32_t* __restrict__ group_start, const int32_t* __restrict__ group_end,
            const int32_t* __restrict__ cands, const int* group_count_ptr, int tile, int max_q,
-           int max_qc, int64_t n_queries, int64_t capacity, int64_t lanes, Meta* meta,
-           int4* __restrict__ items) {
+           int max_qc, int64_t n_queries, int64_t capacity, float typical_scale,
+           float share_scale, Meta* meta, int4* __restrict__ items) {
   chain_wait();
   int* n_items = &meta->n_items;
   int* status = &meta->status;
-  const double pairs = static_cast<double>(meta->pair_total);
-  const int64_t typical = static_cast<int64_t>(1.5 * pairs / static_cast<double>(n_queries));
-  const int64_t share = static_cast<int64_t>(pairs / static_cast<double>(lanes));
+  const float pairs = static_cast<float>(meta->pair_total);
+  const float typical = pairs * typical_scale, share = pairs * share_scale;
   __shared__ uint32_t s_count[8];
   __shared__ uint32_t s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -228,6 +235,10 @@ int64_t resident_warps() {
   return static_cast<int64_t>(sms) * 20;
 }
 
+// Only calls of a full item's worth of queries per warp cut chunked items by
+// their share of the work (chunked_queries).
+bool pairs_wanted(int64_t n_queries) { return n_queries >= resident_warps() * 32; }
+
 // Queries per chunked item (a group whose candidates exceed a tile: every
 // query scans many of them).  An item of q queries gives each query 32 / q
 // lanes.  A problem with fewer than 32 queries per resident query warp is
@@ -253,12 +264,13 @@ int launch_items(const int2* runs, const int32_t* group_start, const int32_t* gr
   const int sblocks = static_cast<int>(sb < 2048 ? sb : 2048);
   if (!cands_ready)  // else the caller's run kernel wrote cands[g] already
     launch_chained(k_group_cands, gblocks, 256, 0, s, runs, group_row, group_count_ptr, cands,
-                   group_start, group_end, meta);
+                   group_start, group_end, pairs_wanted(n_queries) ? 1 : 0, meta);
   const int64_t capacity = static_cast<int64_t>(items_capacity(max_groups, n_queries));
   const int64_t warps = resident_warps();
   launch_chained(k_pack, sblocks, 256, 0, s, group_start, group_end, cands, group_count_ptr, tile,
                  item_query_cap(n_queries), chunked_query_cap(n_queries, warps), n_queries, capacity,
-                 warps > 0 ? warps * 32 : 1, meta, items);
+                 n_queries > 0 ? 1.5f / static_cast<float>(n_queries) : 0.f,
+                 warps > 0 ? 1.f / static_cast<float>(warps * 32) : 1.f, meta, items);
   return cands_ready ? 1 : 2;
 }
 
