@@ -50,3 +50,14 @@ def test_many_clouds(clouds):
     counts = rng.integers(1, 20, clouds)
     xyz = (rng.random((counts.sum(), 3)) * rng.choice([1, 1, 1, 9], counts.sum())[:, None])
     _check(np.ascontiguousarray(xyz, dtype=np.float32), np.cumsum(counts).astype(np.int64), 4)
+
+
+@pytest.mark.parametrize("queries", [1, 63, 64, 65, 95, 96, 2000, 12001, 50000])
+def test_groups_of_many_queries(queries):
+    """A query cell that fills several items by itself, beside cells that share
+    items: the line at two items, remainders, item sizes from 4 to 32."""
+    rng = np.random.default_rng(queries)
+    xyz = _points(rng, 60)
+    many = np.concatenate([rng.random((queries, 3)), _points(rng, 30)]).astype(np.float32)
+    rng.shuffle(many)
+    _check(xyz, np.array([len(xyz)]), 5, np.ascontiguousarray(many), np.array([len(many)]))
