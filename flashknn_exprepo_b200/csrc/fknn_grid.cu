@@ -39,6 +39,8 @@
 // only shortens the keys; it changes neither the cells nor their adjacency.
 #include <climits>
 
+#include <algorithm>
+
 #include "fknn_common.cuh"
 #include "fknn_internal.h"
 #include "fknn_sort.cuh"
@@ -127,8 +129,11 @@ __global__ void __launch_bounds__(256)
   const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (t < sizeof(Meta) / sizeof(int)) reinterpret_cast<int*>(meta)[t] = 0;
-  for (size_t i = t; i < static_cast<size_t>(n_clouds) * 6; i += stride)
-    bbox[i] = (i % 6) < 3 ? INT_MAX : INT_MIN;
+  for (size_t c = t; c < static_cast<size_t>(n_clouds); c += stride) {
+    int* box = bbox + 6 * c;
+    box[0] = box[1] = box[2] = INT_MAX;
+    box[3] = box[4] = box[5] = INT_MIN;
+  }
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   for (size_t i = t; i < slots; i += stride) table[i] = zero;
   for (size_t i = t; i < slots2; i += stride) table2[i] = zero;
@@ -817,7 +822,12 @@ int run_fused(const FusedArgs& f, void* ws, size_t ws_bytes, const QueryShape& s
   const bool qtable = kind == FKNN_QUERY_GENERAL && m > 0;
   const size_t slots = n > 0 ? static_cast<size_t>(b.hash_cap) : 0;
   const size_t qslots = qtable ? static_cast<size_t>(b.qhash_cap) : 0;
-  launch_chained(k_init, capped_blocks(static_cast<int64_t>(slots + qslots) / 4 + 1), 256, 0, s,
+  // Four table slots or one cloud per thread.  Where ids come with the points
+  // n_clouds is their bound (32,768), however few the points: with threads for
+  // the slots alone 300 points took 23 us here.
+  const int64_t init_threads =
+      std::max(static_cast<int64_t>(slots + qslots) / 4 + 1, n_clouds);
+  launch_chained(k_init, capped_blocks(init_threads), 256, 0, s,
                  b.meta, b.bbox, n_clouds, reinterpret_cast<uint4*>(b.hslots), slots,
                  reinterpret_cast<uint4*>(b.qslots), qslots);
   ++nl;

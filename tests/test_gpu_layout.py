@@ -61,3 +61,26 @@ def test_groups_of_many_queries(queries):
     many = np.concatenate([rng.random((queries, 3)), _points(rng, 30)]).astype(np.float32)
     rng.shuffle(many)
     _check(xyz, np.array([len(xyz)]), 5, np.ascontiguousarray(many), np.array([len(many)]))
+
+
+@pytest.mark.parametrize("n", [1, 31, 300, 5000])
+def test_few_points_with_ids_up_to_their_bound(n):
+    """Cloud ids that come with the points are bounded by 32,768 however few
+    the points: every box is emptied, also after a call that filled them."""
+    import flashknn_exprepo_b200 as fk
+    rng = np.random.default_rng(n)
+    for ids in (np.arange(32768), rng.choice([0, 1, 1023, 1024, 20000, 32767], n)):
+        m = len(ids)
+        grid = rng.integers(-40, 40, (m, 3)).astype(np.int64)
+        xyz = (grid + rng.random((m, 3))).astype(np.float32)
+        order = np.argsort(ids, kind="stable")
+        clouds = np.cumsum(np.bincount(ids, minlength=32768)).astype(np.int64)
+        oi, od = O.knn_offsets(xyz[order], clouds, 4, 1.0, 3)
+        to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+        gi, gd = fk.ops.knn_grid(to(xyz), to(np.floor(xyz).astype(np.int64)),
+                                 to(ids.astype(np.int64)), 4, 3, validate=True)
+        dist = gd.cpu().numpy()[order]
+        assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
+        rank = np.empty(m, np.int64)
+        rank[order] = np.arange(m)
+        assert np.array_equal(rank[gi.cpu().numpy()[order]], oi)
