@@ -268,6 +268,68 @@ __device__ __forceinline__ void merge_block(uint32_t (&L)[KCAP], const uint32_t 
   }
 }
 
+// Adds the candidates of one truncated distance, srt[0, end), to the list by
+// their exact keys: the repair of an ambiguous k-th entry (select_blocks).  32
+// positions are tested first, then every lane inserts its own next member, so
+// the insertions number the largest lane's members instead of one for every
+// candidate that some lane of the warp takes.  Where every query is such a
+// one (a lattice of 262 thousand points, 216 candidates) the call takes 197 us
+// at K=16 and 815 at K=64, inserting as the scan meets members 272 and 1747.
+// A second pass of the block selection over the class, with whole keys,
+// took 199 and 1127.
+template <int KCAP, typename DistBits>
+__device__ __forceinline__ void add_class(uint64_t (&E)[KCAP], const uint16_t* srt, int end,
+                                          uint32_t cls, uint32_t pos_mask, uint32_t cut_lim,
+                                          const DistBits& dist_bits) {
+#pragma unroll 1
+  for (int t0 = 0; __any_sync(kFull, t0 < end); t0 += 32) {
+    uint32_t hits = 0u;  // members among srt[t0, t0 + 32)
+#pragma unroll 1
+    for (int h = 0; h < 32 && t0 + h < end; h += 8) {
+      const uint4 p = *reinterpret_cast<const uint4*>(srt + t0 + h);
+      const uint32_t pw[4] = {p.x, p.y, p.z, p.w};
+      uint32_t m = 0u;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float4 c;
+        const uint32_t d = dist_bits((u & 1) ? pw[u >> 1] >> 16 : pw[u >> 1] & 0xffffu, c);
+        if (d <= cut_lim && (d & ~pos_mask) == cls) m |= 1u << u;
+      }
+      hits |= m << h;
+    }
+    while (__any_sync(kFull, hits != 0u)) {
+      uint64_t x = kEmpty;
+      if (hits) {
+        float4 c;
+        const uint32_t d = dist_bits(srt[t0 + __ffs(hits) - 1], c);
+        x = make_key(__uint_as_float(d), c.w);
+        hits &= hits - 1u;
+      }
+      list_insert<KCAP>(E, x);
+    }
+  }
+}
+
+// The same out of line, the list in local memory, so that its registers do not
+// add to the scan's: lists of 64 took 602 us inline over 262 thousand points
+// without ties, 529 so; short lists gain nothing from it.
+template <int KCAP>
+__device__ __noinline__ void add_class_apart(uint64_t* list, const float4* tile,
+                                             const uint16_t* srt, int end, uint32_t cls,
+                                             uint32_t pos_mask, uint32_t cut_lim, float qx,
+                                             float qy, float qz) {
+  auto dist_bits = [&](uint32_t pos, float4& c) {
+    c = tile[pos];
+    return __float_as_uint(sq_dist(c.x, c.y, c.z, qx, qy, qz));
+  };
+  uint64_t E[KCAP];
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) E[j] = list[j];
+  add_class<KCAP>(E, srt, end, cls, pos_mask, cut_lim, dist_bits);
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) list[j] = E[j];
+}
+
 // The lane's KCAP smallest candidates as exact keys (distance bits << 32 |
 // index), ascending; entries from k on may be left out.
 //
@@ -292,7 +354,8 @@ template <int KCAP, typename DistBits>
 __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGroup& g, int k,
                                               uint32_t pos_mask, uint32_t cut_lim,
                                               DistBits& dist_bits, const QueryLaunch& a,
-                                              int n_items, uint32_t none, NextItem& next) {
+                                              int n_items, uint32_t none, NextItem& next,
+                                              const float4* tile, const float4& q) {
   constexpr int B = KCAP <= 16 ? 8 : 16;
   constexpr int M = KCAP < B ? KCAP : B;  // of a block that the list can take
   const uint16_t* srt = g.srt;
@@ -363,14 +426,15 @@ __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGro
   }
   if (__any_sync(kFull, ambiguous)) {
     const int end = ambiguous ? stop : 0;
-    for (int t = 0; __any_sync(kFull, t < end); ++t) {
-      uint64_t x = kEmpty;
-      if (t < end) {
-        float4 c;
-        const uint32_t d = dist_bits(srt[t], c);
-        if (d <= cut_lim && (d & ~pos_mask) == limit) x = make_key(__uint_as_float(d), c.w);
-      }
-      if (__any_sync(kFull, x != kEmpty)) list_insert<KCAP>(E, x);
+    if constexpr (KCAP <= 16) {
+      add_class<KCAP>(E, srt, end, limit, pos_mask, cut_lim, dist_bits);
+    } else {
+      uint64_t list[KCAP];
+#pragma unroll
+      for (int j = 0; j < KCAP; ++j) list[j] = E[j];
+      add_class_apart<KCAP>(list, tile, srt, end, limit, pos_mask, cut_lim, q.x, q.y, q.z);
+#pragma unroll
+      for (int j = 0; j < KCAP; ++j) E[j] = list[j];
     }
   }
 }
@@ -881,7 +945,7 @@ __device__ __forceinline__ void packed_item(const QueryLaunch& a, const int4& it
   uint64_t L[KCAP];
   const uint32_t none = static_cast<uint32_t>(w.T) * 0x10001u;  // the tile's empty record
   select_blocks<KCAP>(L, mine, k, w.T <= 512 ? 511u : 1023u, cut_lim, dist_bits, a, n_items, none,
-                      next);
+                      next, tile, q);
   next.load_groups(a, n_items, n_groups);
   if (lane < qn && mapped) write_row<IdxT, KCAP, EXACT>(a, L, __float_as_int(q.w), k);
   __syncwarp();

@@ -76,3 +76,17 @@ def test_ball_padding_on_both_sides_of_its_radius_rule(radius):
     want_idx, d2 = fk.ops.ball_query_offsets(xyz, offs, 24, radius, radius / 4, 2, None, None)
     assert torch.equal(idx, want_idx) and bool((idx < 0).any()) and bool((idx >= 0).any())
     assert torch.equal(dist, torch.where(idx < 0, torch.full_like(d2, 1e5), torch.sqrt(d2)))
+
+
+@pytest.mark.parametrize("copies", [31, 33, 70])
+@pytest.mark.parametrize("k", [1, 5, 8, 16, 17, 32, 50, 64])
+def test_many_equal_points(k, copies):
+    """Points repeated more often than a test step holds positions: a class of
+    equal distances spans several steps, some lanes' classes more than others'."""
+    rng = np.random.default_rng(copies)
+    base = np.stack(np.meshgrid(np.arange(9), np.arange(9), [0.0], indexing="ij"), -1)
+    xyz = np.repeat((base.reshape(-1, 3) * 3.0 + 0.5).astype(np.float32), copies, 0)
+    xyz[::7] += np.float32(1e-6)
+    rng.shuffle(xyz)
+    _check(np.ascontiguousarray(xyz), k, 0.5)
+    _check(np.ascontiguousarray(xyz), k, 0.8)
