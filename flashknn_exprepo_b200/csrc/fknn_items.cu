@@ -18,13 +18,17 @@
 // queries.  With this and three launches fewer in the construction the whole
 // call takes 71 instead of 87 us on the cube (16 thousand queries, issued
 // back to back) and 557 instead of 574 us on 1.46 million.
+#include <climits>
+
 #include "fknn_common.cuh"
 #include "fknn_internal.h"
 
 namespace fknn {
 
 // cands[g] = number of candidate records of group g (sum of its 27 runs);
-// a group without candidates sets kStatusNoCandidates.  meta->pair_total
+// a group without candidates sets kStatusNoCandidates; a sum beyond 32 bits is
+// reported and counts as none, which the query kernel's own sum then meets as
+// an overfull tile.  meta->pair_total
 // receives the sum of queries x candidates (one atomic per block)
 // where it is wanted (pairs_wanted).
 __global__ void __launch_bounds__(256)
@@ -40,9 +44,14 @@ __global__ void __launch_bounds__(256)
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t row = group_row ? group_row[g] : g;
     const int2* r = runs + row * kNeighbours;
-    int total = 0;
+    int64_t sum = 0;
 #pragma unroll
-    for (int j = 0; j < kNeighbours; ++j) total += max(r[j].y, 0);
+    for (int j = 0; j < kNeighbours; ++j) sum += max(r[j].y, 0);
+    if (sum > INT_MAX) {  // caller tables only: cells do not overlap
+      raise_status(&meta->status, kStatusTable);
+      sum = 0;
+    }
+    const int total = static_cast<int>(sum);
     cands[g] = total;
     if (pairs)
       my_pairs += static_cast<unsigned long long>(total) * max(group_end[g] - group_start[g], 0);

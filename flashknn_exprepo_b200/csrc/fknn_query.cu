@@ -804,6 +804,9 @@ __device__ __forceinline__ int stage_item(const QueryLaunch& a, const NextItem& 
     int len = 0;
     if (gb_ > ga_ && !overflow) {
       run = checked_run(a, run);
+      // A tile is full long before 27 runs of the support's size could wrap the
+      // sum (caller tables over 80 million points).
+      run.y = min(run.y, T + 1);
       const int incl = warp_inclusive_scan(run.y);
       const int first = incl - run.y;
       len = __shfl_sync(kFull, incl, 31);
