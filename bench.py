@@ -168,8 +168,8 @@ def profiled_traffic(k):
 
 
 def profiled_limiter(k):
-    """The unit that bounds the query kernel, from the same ncu summary: the
-    kernel is instruction-bound (ALU pipe), so the HBM fraction alone does
+    """What bounds the query kernel, from the same ncu summary: instruction
+    issue (the ALU pipe is its busiest unit), so the HBM fraction alone does
     not describe it."""
     import re
     path, text = _query_profile(k)
@@ -180,7 +180,7 @@ def profiled_limiter(k):
     per_q = re.search(r"~([0-9]+) warp instructions per query", text)
     if not (alu and issue and per_q):
         return None
-    return {"unit": "ALU pipe (integer compare/select)",
+    return {"unit": "instruction issue",
             "alu_pipe_active_pct": float(alu.group(1)),
             "issue_active_pct": float(issue.group(1)),
             "warp_instructions_per_query": int(per_q.group(1)),
