@@ -304,7 +304,7 @@ __device__ __forceinline__ int axis_offset(int position) {
 // ------------------------------------------------------- cell hash table
 // Open addressing over the support cells (linear probing, capacity >= 2n, so
 // the load stays <= 1/2 whatever the cell count).  A slot holds key + 1 (0 =
-// empty, so the whole table clears with one memset) and the cell's run
+// empty, so k_init clears the table by zeroing it) and the cell's run
 // (start, count): a neighbour lookup is one 16-byte load.
 //
 // The table also builds the cells, as a counting sort by cell instead of a
@@ -691,8 +691,6 @@ struct Bufs {
   uint32_t* slot_of;    // per point: cell slot (support, then general queries)
   uint32_t* rank_of;    // per point: rank inside its cell
   uint32_t* cell_slot;  // per cell / query group id: its slot
-  uint32_t* tile_counts;
-  uint32_t* tile_counts2;
   float4* srec;
   float4* qrec;
   int32_t* pos_of;
@@ -710,6 +708,8 @@ struct Bufs {
   HashSlot* hslots;
   int64_t hash_cap;
   uint32_t* slot_cell;  // cell id of each occupied slot (selected queries)
+  uint32_t* tile_counts;   // non-empty cells and queries per 2,048 cells (selected queries)
+  uint32_t* tile_counts2;
   uint32_t* qcount;     // selected queries per support cell
   uint32_t* qstart;     // first query record of each support cell
   HashSlot* qslots;     // query-cell table (general queries)
@@ -728,8 +728,6 @@ Bufs layout(void* ws, int64_t n, int64_t m, int64_t n_clouds, int kind, size_t* 
   b.slot_of = a.take<uint32_t>(nm);
   b.rank_of = a.take<uint32_t>(nm);
   b.cell_slot = a.take<uint32_t>(nm);
-  b.tile_counts = a.take<uint32_t>(static_cast<size_t>(ceil_div(nm > 0 ? nm : 1, 256)));
-  b.tile_counts2 = a.take<uint32_t>(static_cast<size_t>(ceil_div(nm > 0 ? nm : 1, 2048)));
   b.srec = a.take<float4>(n);
   b.cell_key = a.take<uint64_t>(n);
   b.cell_start = a.take<int32_t>(n);
@@ -741,6 +739,9 @@ Bufs layout(void* ws, int64_t n, int64_t m, int64_t n_clouds, int kind, size_t* 
     b.pos_of = a.take<int32_t>(n);
     b.cell_of = a.take<int32_t>(n);
     b.slot_cell = a.take<uint32_t>(b.hash_cap);
+    const size_t tiles = static_cast<size_t>(ceil_div(n > 0 ? n : 1, 2048));
+    b.tile_counts = a.take<uint32_t>(tiles);
+    b.tile_counts2 = a.take<uint32_t>(tiles);
     b.qcount = a.take<uint32_t>(n);
     b.qstart = a.take<uint32_t>(n);
   }

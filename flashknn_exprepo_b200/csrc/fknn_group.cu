@@ -5,9 +5,9 @@
 //
 // Forward: out[i, j, :] = [xyz[t] - new_xyz[i] | feat[t]] for t = idx[i, j]
 // (the xyz part only with with_xyz); an index below 0 is padding and gives a
-// zero row.  Threads run flat over the output words (float4 when the rows
-// allow it), so every warp stores one contiguous run: a bandwidth-bound copy
-// whose only re-read is the gathered feature row, served from L2 for the
+// zero row.  Every warp stores contiguous runs (rows of float4s, rows staged in
+// shared memory or single words, by width and row count): a bandwidth-bound
+// copy whose only re-read is the gathered feature row, served from L2 for the
 // rows that neighbours share.
 //
 // Backward: grad_feat[t] = sum of grad_out[i, j, feat part] over the entries

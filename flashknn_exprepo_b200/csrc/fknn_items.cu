@@ -295,7 +295,7 @@ int launch_items(const int2* runs, const int32_t* group_start, const int32_t* gr
 }
 
 size_t items_capacity(int64_t max_groups, int64_t n_queries) {
-  // every group yields at most ceil(q/32) + 1 items; every item holds >= 1 query
+  // every item holds at least one query, and no query is in two
   const int64_t a = n_queries + max_groups + 32;
   return static_cast<size_t>(a);
 }

@@ -10,17 +10,17 @@
 // Execution model (B200-first, not the reference's block-per-parent loop):
 //   * persistent CTAs; each warp pulls work items from a device queue
 //     (atomicAdd on Meta::queue_head);
-//   * packed item: up to 32 consecutive queries from up to 32 consecutive
+//   * packed item: up to 32 consecutive queries from up to 16 consecutive
 //     groups, one query per lane.  Each group's 27 runs are staged into the
 //     warp's shared-memory tile, one 16-byte cp.async per record (the runs
 //     are short: a bulk copy each, issued lane after lane, took longer).
-//     Each group's candidates are then
-//     counting-sorted (32 buckets of squared distance) by distance to the
-//     centre of the group's queries, so every lane meets near candidates
-//     first and stops at the first bucket whose lower distance bound exceeds
-//     its current K-th distance (triangle inequality, with a safety margin
-//     for FP32 rounding).  The candidates are taken in blocks, sorted and
-//     merged into the lane's list as 32-bit keys (select_blocks);
+//     Each group's candidates are then counting-sorted (32 buckets of squared
+//     distance) by distance to the centre of the group's queries, so every
+//     lane meets near candidates first and stops at the first bucket whose
+//     lower distance bound exceeds its current K-th distance (triangle
+//     inequality, with a safety margin for FP32 rounding).  The candidates
+//     are taken in blocks, sorted and merged into the lane's list as 32-bit
+//     keys (select_blocks);
 //   * chunked item: one group with more candidates than a tile; G lanes per
 //     query split its candidates, streamed tile by tile by non-multicast
 //     cp.async.bulk copies on the warp's mbarrier, and the G partial
