@@ -336,20 +336,20 @@ __device__ __noinline__ void add_class_apart(uint64_t* list, const float4* tile,
 // Bound by instruction issue.  The scan sorts blocks of B candidates as
 // 32-bit keys and merges each block into the list (a minimum and a maximum
 // per compare-exchange), in place of one warp-wide 64-bit insertion per
-// accepted candidate of any lane: 309 -> 190 warp instructions per query at
+// accepted candidate of any lane: 309 -> 180 warp instructions per query at
 // K=16.  The first block goes through the same loop as the rest (no
 // separate fill): the code the warps share has to stay small, since straight
 // copies of it made instruction fetch the first stall (2.8 of 10 cycles per
-// instruction).  With staging and sort the whole call over the 16-cloud batch
-// (1.46 million queries, K=16) went from 861 to 574 us, over 700 thousand
-// queries at K=32 from 880 to 484 us, over 300 thousand at K=64 from 1182 to
-// 522 us.  Short lists gain the same way: 300 thousand queries at K=3 125 ->
-// 100 us, 700 thousand at K=1 323 -> 307 us.  The keys
-// drop the low 9 or 10 bits of the distance, so the exact keys of the list
+// instruction).  With the staging, the sort and a shorter construction the
+// whole call over the 16-cloud batch (1.46 million queries, K=16) went from
+// 861 to 553 us, over 700 thousand queries at K=32 from 880 to 476 us, over 300
+// thousand at K=64 from 1182 to 455 us.  Short lists gain the same way: 300
+// thousand queries at K=3 125 -> 98 us, 700 thousand at K=1 323 -> 302 us.  The
+// keys drop the low 9 or 10 bits of the distance, so the exact keys of the list
 // are computed at the end and neighbours that the truncation left in the
 // wrong order are exchanged; a lane whose k-th entry shares its truncated
 // distance with a candidate it left out collects the candidates of that one
-// truncated distance again, with exact keys.
+// truncated distance again, with exact keys (add_class).
 template <int KCAP, typename DistBits>
 __device__ __forceinline__ void select_blocks(uint64_t (&E)[KCAP], const LaneGroup& g, int k,
                                               uint32_t pos_mask, uint32_t cut_lim,
